@@ -8,19 +8,10 @@
 // Each point may use phases set earlier in the same ring, so the walk is a
 // serial chain.  Most of a point's pairs, though, read phases that were final
 // long before: a pair is "recent" only when u or v was visited within the
-// kRecoLag visits before w (the arc of the ring just behind w).  The walk is
-// therefore split:
-//   - summing warps form, for visit q, the sum over its non-recent pairs as
-//     soon as the walk has passed q - kRecoLag, eight pair slots per lane at a
-//     time so that the plan, flag and phase gathers overlap;
-//   - one serial warp runs the visits in order and adds only the recent pairs (a list
-//     of at most kRecentMax per visit, prefetched with the plan phasors) to
-//     that share, then sets the point's phase and flag.
-// Which pairs are recent depends only on the visit list (per point: its visit
-// indices), so it is computed in parallel before the walk.
-// Depths below kClusterDepth walk in one CTA (phase_pipe_kernel); deeper
-// bispectra, whose (d+1)^2 pairs per visit one CTA's summing warps cannot
-// keep up with, walk in a thread-block cluster (phase_cluster_kernel).
+// kRecoLag visits before w (the arc of the ring just behind w; at most 64
+// pairs, a fact of the lag).  Which pairs are recent depends only on the visit
+// list, so spiral_plan_kernel lists them ahead of the walk with everything
+// else that does not depend on the chain; phase_walk_kernel is the walk.
 //
 // Precision: per-pair products in FP32 from an FP32 mirror of the phase map
 // (~1e-7 rad per pair); the non-recent share is summed in FP32 per lane and in
@@ -36,6 +27,7 @@
 namespace smip_gpu {
 
 constexpr int kRecoThreads = 512;
+constexpr int kMaxWords = (65 * 65 + 31) / 32; // words of a pair-slot mask at the largest depth
 
 __device__ __forceinline__ int wrap_idx(int x, int y, int W, int H)
 {
@@ -76,12 +68,30 @@ __device__ __forceinline__ void ff_add(float& hi, float& lo, float bh, float bl)
     lo = __fsub_rn(e, __fsub_rn(hi, s));
 }
 
+// phi(u) phi(v) conj(b), every rounding spelt out: a visit's terms are formed in
+// several places, and the compiler may contract the same expression differently
+// in each.
+__device__ __forceinline__ float2 pair_product(float2 u, float2 v, float bx, float by)
+{
+    const float2 m = make_float2(__fmaf_rn(u.x, v.x, -__fmul_rn(u.y, v.y)), __fmaf_rn(u.y, v.x, __fmul_rn(u.x, v.y)));
+    return make_float2(__fmaf_rn(m.x, bx, __fmul_rn(m.y, by)), __fmaf_rn(m.y, bx, -__fmul_rn(m.x, by)));
+}
+// For normal arguments, 0 and NaN: rsqrtf without its scaling of subnormals.
+__device__ __forceinline__ float rsqrt_ftz(float x)
+{
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float norm2(float2 p) { return __fmaf_rn(p.x, p.x, __fmul_rn(p.y, p.y)); }
+
 // ----------------------------------------------------------------- plan
 // The bispectrum side of every pair the walk can use depends only on (w, v),
 // not on the chain: plan[q][t] = unit phasor of B(w_q - v_t, v_t), or
 // (0, 0) when the pair never contributes (u outside the map, |B| <= eps,
 // w skipped by calc_phase), or NaN where Bispectrum::get_element would throw.
-// Fully parallel over (visit, v); the serial chain then only streams rows.
+// Fully parallel over (visit, v).  (The ring-parallel estimator's; the spiral
+// walk's plan, with its recent pairs taken out, is spiral_plan_kernel's.)
 __global__ void __launch_bounds__(256) reco_plan_kernel(const RecoJob* __restrict__ jobs)
 {
     const RecoJob J = jobs[blockIdx.y];
@@ -128,66 +138,96 @@ __global__ void __launch_bounds__(256) reco_plan_kernel(const RecoJob* __restric
     }
 }
 
-// ------------------------------------------------------ pipelined walk
-// A visit's pairs split by when their phases became final.  A pair (u, v)
-// of visit q is "recent" when u or v was visited within the kRecoLag visits
-// before q (visit lists per point: pvis); every other pair only reads phases
-// and flags that no visit in [q - kRecoLag, q) can change, so its share of
-// the sum can be formed as soon as the walk has passed q - kRecoLag.  The
-// serial part of a visit is then the few recent pairs (the arc of the current
-// ring just behind w) instead of all (d+1)^2.
-__device__ __forceinline__ bool visited_in_lag(int4 pv, int q)
-{
-    if (pv.w > 3) // more visits than recorded: treat as recent
-        return true;
-    const int lo = q - kRecoLag;
-    return (pv.x >= 0 && pv.x >= lo && pv.x < q) || (pv.y >= 0 && pv.y >= lo && pv.y < q)
-           || (pv.z >= 0 && pv.z >= lo && pv.z < q);
-}
+// ----------------------------------------------------------- the spiral
+// The walk's inputs that do not depend on the chain, one warp per visit q:
+//   plan[q][t]: the unit phasor of B(w - v_t, v_t) of every non-recent pair,
+//     or NaN for a pair that the sum leaves out (u outside the map, |B| <= eps,
+//     a recent pair), so that one test of the product tells a usable pair;
+//   rec[q][64]: the recent pairs in increasing slot order (at most 32 by u and
+//     32 by v): phasor, slot and the ages ku, kv (q - the last visit of u, v
+//     within the lag; 0: none);
+//   meta[q]: the point's place in the padded map (-1: outside), its FFT-order
+//     index, the number of recent pairs, the age of the point's own last visit
+//     within the lag, and its slot when it lies in the v box.
+// A visit with at most 32 recent pairs of which at most one has age 1 is
+// "fast": its list is stored permuted by XOR with that pair's position, which
+// puts the pair into lane 0 and leaves the order of a butterfly sum as it is.
+// A phasor that is NaN (Bispectrum::get_element would throw, or B is not a
+// number) has the payload kOorBits and raises J.oor.
+// Bound by the scattered reads of B (one 32-byte sector per pair): 64 M pairs
+// at 256 x 256, d = 32.
+constexpr unsigned kUnusable = 0x7fc00000u;
+constexpr unsigned kOorBits = 0x7fc00001u;
+constexpr int kPlanWarps = 8;
 
-__global__ void __launch_bounds__(256) reco_recent_kernel(const RecoJob* __restrict__ jobs)
+// rec code: slot t (13 bits) | ku << 13 | kv << 19 | phasor is kOorBits << 25
+// meta.z: recent pairs | kc << 8 | fast << 16 | runnable << 17
+__global__ void __launch_bounds__(32 * kPlanWarps) spiral_plan_kernel(const RecoJob* __restrict__ jobs)
 {
+    extern __shared__ int slot_xy[]; // [nwords * 32] vx | vy << 16
+    __shared__ unsigned mask_s[kPlanWarps][kMaxWords];
+    __shared__ unsigned short list_s[kPlanWarps][kRecentMax];
+    __shared__ unsigned code_s[kPlanWarps][kRecentMax];
     const RecoJob J = jobs[blockIdx.y];
-    const int W = J.W, H = J.H, De = J.De;
-    const int nside = De + 1, nv = nside * nside, nwords = (nv + 31) / 32;
+    const int W = J.W, H = J.H, De = J.De, e = De / 2;
+    const int nside = De + 1, nv = nside * nside, nwords = (nv + 31) / 32, row = nwords * 32;
+    for (int t = threadIdx.x; t < row; t += blockDim.x) {
+        const int vx = -e + t % nside, vy = -e + t / nside;
+        slot_xy[t] = (int)(((unsigned)vx & 0xffffu) | ((unsigned)vy << 16));
+    }
+    __syncthreads();
+    BispecDims d;
+    const int szW = (W / 2) * 2 + 1, szH = (H / 2) * 2 + 1, szD = De + 1;
+    d.sizes[0] = szW; d.sizes[1] = szH; d.sizes[2] = szD; d.sizes[3] = szD;
+    d.base[0] = szW - szW / 2; d.base[1] = szH; d.base[2] = szD - szD / 2; d.base[3] = szD;
+    for (int n = 0; n < 4; ++n) {
+        d.mn[n] = -(d.sizes[n] / 2);
+        d.mx[n] = d.sizes[n] + d.mn[n] - 1;
+    }
+    d.base_size = (long long)d.base[0] * d.base[1] * d.base[2] * d.base[3];
     const int pmin0 = -(W >> 1), pmin1 = -(H >> 1);
     const int pmax0 = -W / 2 + W - 1, pmax1 = -H / 2 + H - 1;
-    const long long total = (long long)J.nvisits * nwords;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-         e += (long long)gridDim.x * blockDim.x) {
-        const int q = (int)(e / nwords), wd = (int)(e - (long long)q * nwords);
+    auto in_map = [&](int x, int y) { return x >= pmin0 && x <= pmax0 && y >= pmin1 && y <= pmax1; };
+    auto pack = [](int x, int y) { return (int)(((unsigned)x & 0xffffu) | ((unsigned)y << 16)); };
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned* mask = mask_s[warp];
+    unsigned short* list = list_s[warp];
+    unsigned* code = code_s[warp];
+    const float2 nan2 = make_float2(__uint_as_float(kUnusable), __uint_as_float(kUnusable));
+    for (int q = blockIdx.x * kPlanWarps + warp; q < J.nvisits; q += gridDim.x * kPlanWarps) {
         const int2 w = J.visits[q];
-        unsigned bits = 0u;
-        if (!(w.x < pmin0 || w.x > pmax0 || w.y < pmin1 || w.y > pmax1)) {
-            for (int b = 0; b < 32; ++b) {
-                const int t = wd * 32 + b;
-                if (t >= nv)
-                    break;
-                const int vx = -De / 2 + t % nside, vy = -De / 2 + t / nside;
-                const int ux = w.x - vx, uy = w.y - vy;
-                if (ux < pmin0 || ux > pmax0 || uy < pmin1 || uy > pmax1)
-                    continue;
-                if (visited_in_lag(J.pvis[wrap_idx(ux, uy, W, H)], q) || visited_in_lag(J.pvis[wrap_idx(vx, vy, W, H)], q))
-                    bits |= 1u << b;
+        if (!in_map(w.x, w.y)) {
+            if (lane == 0)
+                J.meta[q] = make_int4(-1, 0, 0, -1);
+            continue;
+        }
+        // lane j: the visit of age j + 1
+        const int pq = q - 1 - lane;
+        int2 pj = make_int2(0, 0);
+        if (pq >= 0)
+            pj = J.visits[pq];
+        const bool inj = pq >= 0 && in_map(pj.x, pj.y);
+        const int pkj = inj ? pack(pj.x, pj.y) : (int)0x80008000; // not a point of any map
+        for (int i = lane; i < nwords; i += 32)
+            mask[i] = 0u;
+        __syncwarp();
+        if (inj) {
+            const int ux = w.x - pj.x, uy = w.y - pj.y; // the pair's other member
+            if (abs(pj.x) <= e && abs(pj.y) <= e && in_map(ux, uy)) { // v = pj
+                const int t = (pj.y + e) * nside + pj.x + e;
+                atomicOr(&mask[t >> 5], 1u << (t & 31));
+            }
+            if (abs(ux) <= e && abs(uy) <= e) { // u = pj
+                const int t = (uy + e) * nside + ux + e;
+                atomicOr(&mask[t >> 5], 1u << (t & 31));
             }
         }
-        J.rbits[e] = bits;
-    }
-}
-
-// One warp per visit: the recent pair slots in increasing order, or -1 when
-// there are more than kRecentMax (the serial warp then takes every pair).
-__global__ void __launch_bounds__(256) reco_rlist_kernel(const RecoJob* __restrict__ jobs)
-{
-    const RecoJob J = jobs[blockIdx.y];
-    const int nv = (J.De + 1) * (J.De + 1), nwords = (nv + 31) / 32;
-    const int lane = threadIdx.x & 31;
-    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
-    for (int q = gw; q < J.nvisits; q += nw) {
-        const unsigned* rb = J.rbits + (long long)q * nwords;
-        int base = 0;
+        __syncwarp();
+        int rc = 0;
         for (int w0 = 0; w0 < nwords; w0 += 32) {
-            const unsigned bits = w0 + lane < nwords ? rb[w0 + lane] : 0u;
+            const unsigned bits = w0 + lane < nwords ? mask[w0 + lane] : 0u;
+            if (!__any_sync(0xffffffffu, bits != 0u))
+                continue;
             const int c = __popc(bits);
             int incl = c; // inclusive prefix over the lanes
 #pragma unroll
@@ -196,62 +236,146 @@ __global__ void __launch_bounds__(256) reco_rlist_kernel(const RecoJob* __restri
                 if (lane >= o)
                     incl += y;
             }
-            int pos = base + incl - c;
-            unsigned b = bits;
-            while (b) {
-                const int k = __ffs(b) - 1;
-                b &= b - 1;
-                if (pos < kRecentMax)
-                    J.rlist[(long long)q * kRecentMax + pos] = (unsigned short)((w0 + lane) * 32 + k);
-                ++pos;
-            }
-            base += __shfl_sync(0xffffffffu, incl, 31);
+            int pos = rc + incl - c;
+            for (unsigned b = bits; b; b &= b - 1)
+                list[pos++] = (unsigned short)((w0 + lane) * 32 + __ffs(b) - 1);
+            rc += __shfl_sync(0xffffffffu, incl, 31);
         }
-        if (lane == 0)
-            J.rcount[q] = base > kRecentMax ? -1 : base;
+        __syncwarp();
+        const int ta = lane < rc ? list[lane] : 0, tb = lane + 32 < rc ? list[lane + 32] : 0;
+        const int va = slot_xy[ta], vb = slot_xy[tb];
+        const int ua = pack(w.x - (short)va, w.y - (va >> 16)), ub = pack(w.x - (short)vb, w.y - (vb >> 16));
+        int kua = 0, kva = 0, kub = 0, kvb = 0;
+        for (int k = 32; k >= 1; --k) { // the smallest age is kept
+            const int p = __shfl_sync(0xffffffffu, pkj, k - 1);
+            kua = p == ua ? k : kua;
+            kva = p == va ? k : kva;
+            kub = p == ub ? k : kub;
+            kvb = p == vb ? k : kvb;
+        }
+        const unsigned late_a = __ballot_sync(0xffffffffu, lane < rc && (kua == 1 || kva == 1));
+        const unsigned late_b = __ballot_sync(0xffffffffu, lane + 32 < rc && (kub == 1 || kvb == 1));
+        const unsigned own = __ballot_sync(0xffffffffu, pkj == pack(w.x, w.y));
+        const int kc = own ? __ffs(own) : 0;
+        const bool fast = rc <= 32 && __popc(late_a) + __popc(late_b) <= 1 && kc == 0;
+        const int perm = fast && late_a ? __ffs(late_a) - 1 : 0;
+        const bool run = abs(w.x) + abs(w.y) > 1; // phasereco.h:84
+        if (lane < rc)
+            code[lane] = (unsigned)(ta | kua << 13 | kva << 19);
+        if (lane + 32 < rc)
+            code[lane + 32] = (unsigned)(tb | kub << 13 | kvb << 19);
+        if (lane == 0) {
+            const int bx = w.x - pmin0 + e, by = w.y - pmin1 + e;
+            const int vs = abs(w.x) <= e && abs(w.y) <= e ? (w.y + e) * nside + w.x + e : -1;
+            J.meta[q] = make_int4(by * (W + De) + bx, wrap_idx(w.x, w.y, W, H),
+                                  rc | kc << 8 | (fast ? 1 << 16 : 0) | (run ? 1 << 17 : 0), vs);
+        }
+        __syncwarp();
+        if (!run)
+            continue;
+        uint4* rec = J.rec + (long long)q * kRecentMax;
+        const uint4 none = make_uint4(kUnusable, kUnusable, 0u, 0u);
+        if (lane >= rc)
+            rec[lane ^ perm] = none;
+        if (rc > 32 && lane + 32 >= rc)
+            rec[lane + 32] = none;
+        float2* prow = J.plan + (long long)q * row;
+        int before = 0; // recent pairs in the words before word i
+        bool oor = false;
+        for (int i = 0; i < nwords; ++i) {
+            const int t = lane + 32 * i;
+            float2 out = nan2;
+            if (t < nv) {
+                const int xy = slot_xy[t];
+                const int vx = (short)xy, vy = xy >> 16;
+                const int ux = w.x - vx, uy = w.y - vy;
+                if (in_map(ux, uy)) {
+                    int cj = 0;
+                    const long long off = bispec_get_offset(d, ux, uy, vx, vy, &cj);
+                    bool bad = off < 0;
+                    if (!bad) {
+                        float2 b = __ldg(&J.B[off]);
+                        if (cj)
+                            b.y = -b.y;
+                        float2 bh;
+                        if (unit_phasor(b, &bh)) {
+                            bad = isnan(bh.x);
+                            out = bh;
+                        }
+                    }
+                    if (bad) {
+                        out = make_float2(__uint_as_float(kOorBits), __uint_as_float(kOorBits));
+                        oor = true;
+                    }
+                }
+            }
+            const unsigned bits = mask[i];
+            if ((bits >> lane) & 1u) {
+                const int pos = before + __popc(bits & ((1u << lane) - 1u));
+                const unsigned c = code[pos] | (__float_as_uint(out.x) == kOorBits ? 1u << 25 : 0u);
+                rec[pos ^ perm] = make_uint4(__float_as_uint(out.x), __float_as_uint(out.y), c, 0u);
+                out = nan2;
+            }
+            before += __popc(bits);
+            prow[t] = out;
+        }
+        if (oor)
+            atomicOr(J.oor, 1);
+        __syncwarp();
     }
 }
 
-// The walk, one thread-block cluster per job.  Warp 0 of the cluster's rank-0
-// CTA runs the visits in order: for visit q it waits for the share of the
-// non-recent pairs, adds the recent pairs (or all pairs when the list
-// overflowed), forms the phase and advances `progress`.  The warps of the
-// other CTAs form the non-recent shares of visits q = g (mod number of such
-// warps), each once progress >= q - kRecoLag, and store them into a ring of
-// kRing slots in rank 0's shared memory.  A visit's share is split into up to
-// kMaxParts parts over ranges of its pair slots, summed by different warps
-// (only the kRecoLag visits ahead of the walk can be summed at any time, so
-// a visit's latency, not the warp count, sets the rate), and the serial warp
-// adds the parts in part order (distributed shared memory: st.async stores that complete
-// the slot's mbarrier, on which the serial warp waits locally).  `progress`
-// is published with a release at cluster scope, so the summing warps, after
-// their acquire, read the phases and flags the walk set from the phase map in
-// global memory, where an unflagged point holds NaN.  Rank 0 keeps its SM
-// for the serial warp (summing warps beside it take its issue slots: 3.4k
-// against 2.3k cycles per visit at 256 x 256, d = 32); a cluster of one CTA
-// (where the GPU cannot place more) sums on its other warps.  Every wait is
-// bounded; on a timeout the walk stops and the error is recorded.
+// The walk: one cluster of CTAs per job (or one CTA, where the GPU places no
+// cluster).
+//   warp 0 of rank 0 (the serial warp) runs the visits in order;
+//   the writer, on another sub-partition, copies what the serial warp found
+//     into the phase map in global memory and publishes the progress to every
+//     CTA;
+//   summing warps form, for visit q, the share of the non-recent pairs once
+//     the progress has reached q - kRecoLag, resolve the recent pairs' members
+//     that lie outside the lag, and post both into slot q mod kRing of rank 0;
+//   gathering warps of rank 0 wait for the other CTAs' posts (st.async, whose
+//     completion the slot's mbarrier counts: a plain store and a release at
+//     cluster scope held the summing warp for 2,200 cycles a visit), add a
+//     visit's parts and set the tag that the serial warp looks at.
+// In a cluster rank 0 sums nothing; in a lone CTA the summing warps are those
+// of the other three SM sub-partitions, so that the serial warp keeps the
+// issue slots of its own.
+//
+// What a visit must wait for is the phase of the visit just before it.  The
+// serial warp therefore does everything else of visit q + 1 while the chain of
+// visit q runs: the terms of the pairs of age >= 2, and their butterfly sum
+// over the lanes, of which lane 0 keeps the sibling sum that it receives at
+// each level.  Lane 0 holds the one pair of age 1: its term, five additions of
+// those sibling sums (bit for bit the butterfly's result), the float-float
+// addition to the share and the phase are the chain, with no shuffle, branch
+// or memory access between two visits.  Visits that are not "fast" (two pairs
+// of age 1, or more than 32 recent pairs: near the origin, 2 % of the visits
+// at 256 x 256) form their sum at once, as 32 or 64 terms.
+//
+// The phase map is kept centred with De / 2 points of padding and holds NaN
+// where there is no phase, so that a pair's u is one address and needs no
+// bounds or flag test: a product with an unflagged or outside point is NaN.
+// Every wait is bounded; on a timeout the walk stops and the error is recorded.
+//
+// Bound by latency: the chain and the early part of one visit, issued by one
+// warp, take 306 cycles on an idle SM; a visit of the walk takes about 450
+// (2,000 before: 256 x 256, d = 32, R = 128 in 14.4 ms instead of 56.9, and
+// 512 x 512, d = 48, R = 200 in 34.7 ms instead of 153.7).
 constexpr int kRing = 64;
-constexpr int kPhaseCache = 2048;
-// CTAs per job (cluster size) from depth kClusterDepth on, fewer where the GPU
-// cannot place 8.  Below it phase_pipe_kernel walks in one CTA: its summing
-// warps keep up with the serial warp (256 x 256, d = 32, R = 128: 58.0 ms in
-// one CTA, 59.4 ms in a cluster), and a cluster would hold 8 SMs instead of 1
-// while it walks, which other jobs sharing the GPU need.
-constexpr int kWalkCtas = 8;
-constexpr int kClusterDepth = 40;
-constexpr uint32_t kShareBytes = sizeof(float4) + sizeof(int); // one part's st.async payload
 constexpr int kMaxParts = 6;
-// static + the largest dynamic shared memory (1024 x 1024 flags, d = 64) fit a CTA's 227 KB
-static_assert(kRing * kMaxParts * (sizeof(float4) + sizeof(int)) + kRing * 8 + kPhaseCache * (sizeof(int) + sizeof(float2))
-                      + 64 + (sizeof(float2) + sizeof(int2)) * 65 * 65 + sizeof(unsigned) * (kMaxSide * kMaxSide / 32)
-                  <= 227 * 1024,
-              "walk shared memory");
+constexpr int kStep = 4;                 // visits between two looks of the serial warp at the other warps
+constexpr int kGroups = kRing / kStep;
+constexpr int kSkip = 0, kFast = 1, kWide = 2; // ctl.z: how the serial warp treats a visit
+constexpr unsigned long long kRecoWaitNs = 2000000000ull;
+static_assert(kRing > kRecoLag + 8, "ring slots outlive the lag and the serial warp's look-ahead");
 
-// parts per visit share: about 16 words of pair slots (512 slots) each
-__host__ __device__ __forceinline__ int share_parts(int nwords)
+// parts per visit share from depth kPartsDepth on: about 16 words of pair
+// slots (512 slots) each, so that a visit's sum is short enough for the lag
+constexpr int kPartsDepth = 40;
+__host__ __device__ __forceinline__ int share_parts(int De, int nwords)
 {
-    const int p = nwords / 16;
+    const int p = De < kPartsDepth ? 1 : nwords / 16;
     return p < 1 ? 1 : (p > kMaxParts ? kMaxParts : p);
 }
 
@@ -262,656 +386,576 @@ __device__ __forceinline__ void st_release_cta(int* p, int v)
 {
     asm volatile("st.release.cta.shared.b32 [%0], %1;" ::"r"(smem_u32(p)), "r"(v) : "memory");
 }
-static_assert(kRing > kRecoLag + 1, "ring slots outlive the lag");
-constexpr unsigned long long kRecoWaitNs = 2000000000ull;
-
-__device__ __forceinline__ bool unflagged(float2 ph) { return isnan(ph.x); }
-
-__global__ void __launch_bounds__(kRecoThreads, 1) phase_cluster_kernel(const RecoJob* __restrict__ jobs)
-{
-    extern __shared__ __align__(16) unsigned char smraw[];
-    __shared__ float4 ring_s[kRing][kMaxParts];
-    __shared__ int ring_n[kRing][kMaxParts];
-    __shared__ __align__(8) uint64_t ring_bar[kRing]; // slot q % kRing: visit q's share has landed
-    __shared__ int progress;
-    __shared__ int abort_walk;
-    __shared__ int pc_key[kPhaseCache];   // serial warp: phases it set, by point
-    __shared__ float2 pc_val[kPhaseCache];
-    const uint32_t rank = cluster_rank(), ncta = cluster_size();
-    const RecoJob J = jobs[blockIdx.x / ncta];
-    const int W = J.W, H = J.H, De = J.De;
-    const int nbits = W * H;
-    const int nside = De + 1, nv = nside * nside, nwords = (nv + 31) / 32;
-    const int nparts = share_parts(nwords);
-    float2* vtab = reinterpret_cast<float2*>(smraw);                        // [nv] phases of the v disc (rank 0)
-    int2* slot_v = reinterpret_cast<int2*>(vtab + nv);                      // [nv] (vx | vy << 16, map index of v)
-    unsigned int* flagbits = reinterpret_cast<unsigned int*>(slot_v + nv);  // [W*H bits] (rank 0)
-    for (int i = threadIdx.x; i < nv; i += blockDim.x) {
-        const int vx = -De / 2 + i % nside, vy = -De / 2 + i / nside;
-        slot_v[i] = make_int2((int)(((unsigned)vx & 0xffffu) | ((unsigned)vy << 16)), wrap_idx(vx, vy, W, H));
-    }
-    if (rank == 0) {
-        for (int i = threadIdx.x; i < (nbits + 31) / 32; i += blockDim.x)
-            flagbits[i] = 0u;
-        for (int i = threadIdx.x; i < nv; i += blockDim.x)
-            vtab[i] = make_float2(0.f, 0.f);
-        if (threadIdx.x == 0) {
-            progress = 0;
-            abort_walk = 0;
-            for (int i = 0; i < kRing; ++i) // one arrival per phase: the serial warp's expect_tx
-                mbar_init(&ring_bar[i], 1);
-            fence_mbar_init();
-        }
-        __syncthreads();
-        if (threadIdx.x < 5) { // seeds (phasereco.h:42-54); all inside the v disc
-            const int sx[5] = { 0, 1, 0, -1, 0 }, sy[5] = { 0, 0, 1, 0, -1 };
-            const int p = wrap_idx(sx[threadIdx.x], sy[threadIdx.x], W, H);
-            const float im = threadIdx.x < 3 ? 0.f : -0.f;
-            J.phf[p] = make_float2(1.f, im);
-            J.sums[p] = make_float4(0.f, 0.f, 0.f, 0.f);
-            J.cnt[p] = -1;
-            vtab[(sy[threadIdx.x] + De / 2) * nside + sx[threadIdx.x] + De / 2] = make_float2(1.f, im);
-            atomicOr(&flagbits[p >> 5], 1u << (p & 31));
-        }
-    }
-    cluster_sync_all(); // rank 0's ring, progress and the seeds are set
-    const int pmin0 = -(W >> 1), pmin1 = -(H >> 1);
-    const int pmax0 = -W / 2 + W - 1, pmax1 = -H / 2 + H - 1;
-    const int szW = (W / 2) * 2 + 1, szH = (H / 2) * 2 + 1;
-    const int umn0 = -(szW / 2), umx0 = szW - szW / 2 - 1, umn1 = -(szH / 2), umx1 = szH - szH / 2 - 1;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t a_abort = dsmem_addr(&abort_walk, 0);
-    const uint32_t a_progress = dsmem_addr(&progress, 0);
-
-    auto flag = [&](int p) { return ((flagbits[p >> 5] >> (p & 31)) & 1u) != 0u; };
-    // bounded wait on a condition; false on a timeout or when another warp
-    // of the cluster gave up (then the walk stops)
-    auto wait_until = [&](auto cond) {
-        if (cond())
-            return true;
-        const unsigned long long t0 = globaltimer_ns();
-        for (;;) {
-            for (int i = 0; i < 64; ++i)
-                if (cond())
-                    return true;
-            if (dsmem_ld_relaxed(a_abort))
-                return false;
-            if (globaltimer_ns() - t0 > kRecoWaitNs) {
-                record_error(J.err, SMIP_DEV_ERR_TIMEOUT);
-                dsmem_st_relaxed(a_abort, 1);
-                return false;
-            }
-        }
-    };
-
-    // Pairs of visit q, eight slots per lane at a time, so that the plan and
-    // phase gathers overlap.  skip_recent leaves the recent pairs out (the
-    // serial warp takes them).  LOCAL: the serial warp's view (flags and v
-    // phases in rank 0's shared memory, u phases from `phase`); otherwise
-    // flags and both phases from the phase map in global memory (NaN: no
-    // phase yet).
-    // Words [wb, we) of the visit's pair slots.
-    auto sum_pairs = [&](int q, int2 w, bool skip_recent, auto local, auto phase, int wb, int we, float& sr, float& si,
-                         int& cnt) {
-        constexpr bool LOCAL = decltype(local)::value;
-        constexpr int kB = 8;
-        const unsigned* rb = J.rbits + (long long)q * nwords;
-        const float2* prow = J.plan + (long long)q * nv;
-        for (int i0 = wb; i0 < we; i0 += kB) {
-            float2 bh[kB], ph[kB], pvv[kB];
-            bool use[kB];
-#pragma unroll
-            for (int k = 0; k < kB; ++k) {
-                const int t = lane + 32 * (i0 + k);
-                use[k] = i0 + k < we && t < nv;
-                // slot t's bit is bit `lane` of word i0 + k
-                if (skip_recent)
-                    use[k] = use[k] && !((rb[i0 + k] >> lane) & 1u);
-                bh[k] = use[k] ? prow[t] : make_float2(0.f, 0.f);
-                if (use[k]) { // the flags and phase gathers do not wait for the plan
-                    const int2 sv = slot_v[t];
-                    const int vx = (int)(short)(sv.x & 0xffff), vy = sv.x >> 16;
-                    const int ux = w.x - vx, uy = w.y - vy;
-                    const bool inu = !(ux < pmin0 || ux > pmax0 || uy < pmin1 || uy > pmax1);
-                    const int pu = inu ? wrap_idx(ux, uy, W, H) : 0, pv = sv.y;
-                    if constexpr (LOCAL) {
-                        use[k] = inu && flag(pu) && flag(pv);
-                        ph[k] = use[k] ? phase(pu) : make_float2(0.f, 0.f);
-                        pvv[k] = vtab[t];
-                    } else {
-                        ph[k] = inu ? J.phf[pu] : make_float2(0.f, 0.f);
-                        pvv[k] = J.phf[pv];
-                        use[k] = inu;
-                    }
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < kB; ++k) {
-                if constexpr (!LOCAL)
-                    use[k] = use[k] && !unflagged(ph[k]) && !unflagged(pvv[k]);
-                if (!use[k] || (bh[k].x == 0.f && bh[k].y == 0.f)) // the plan's zero: never contributes
-                    continue;
-                if (isnan(bh[k].x)) {
-                    record_error(J.err, SMIP_DEV_ERR_OUT_OF_RANGE);
-                    continue;
-                }
-                const float2 p = cmul(cmul(ph[k], pvv[k]), make_float2(bh[k].x, -bh[k].y));
-                const float r = rsqrtf(p.x * p.x + p.y * p.y);
-                sr += p.x * r;
-                si += p.y * r;
-                ++cnt;
-            }
-        }
-    };
-    using Local = std::true_type;
-    using Global = std::false_type;
-
-    if (rank == 0 && warp == 0) {
-        // ------------------------------------------------ serial warp
-        // Visit data that does not depend on the walk is loaded ahead: the
-        // visit, its recent-pair count and slots two visits ahead, their plan
-        // phasors one visit ahead.  Phases the walk just set come from a
-        // shared-memory cache keyed by point (a miss reads the phase map).
-        for (int i = lane; i < kPhaseCache; i += 32)
-            pc_key[i] = -1;
-        __syncwarp();
-        struct Ahead {
-            int2 w;
-            int rc, ta, tb;
-            float2 ba, bb;
-        };
-        // the list slots are loaded without waiting for the count (a visit's
-        // kRecentMax entries are always allocated) and masked one visit later
-        auto load_meta = [&](int q, Ahead& a) {
-            if (q >= J.nvisits)
-                return;
-            a.w = J.visits[q];
-            a.rc = J.rcount[q];
-            const unsigned short* rl = J.rlist + (long long)q * kRecentMax;
-            a.ta = rl[lane];
-            a.tb = rl[lane + 32];
-        };
-        auto load_plan = [&](int q, Ahead& a) {
-            if (q >= J.nvisits)
-                return;
-            a.ta = lane < a.rc ? a.ta : -1;
-            a.tb = lane + 32 < a.rc ? a.tb : -1;
-            const float2* prow = J.plan + (long long)q * nv;
-            a.ba = a.ta >= 0 ? prow[a.ta] : make_float2(0.f, 0.f);
-            a.bb = a.tb >= 0 ? prow[a.tb] : make_float2(0.f, 0.f);
-        };
-        // every slot expects its first visit's share (visits 0 .. kRing-1)
-        if (lane == 0)
-            for (int i = 0; i < kRing; ++i)
-                mbar_arrive_expect_tx(&ring_bar[i], kShareBytes * nparts);
-        Ahead c0 {}, c1 {}, c2 {};
-        load_meta(0, c0);
-        load_plan(0, c0);
-        load_meta(1, c1);
-        auto phase_of = [&](int p) {
-            const int h = p & (kPhaseCache - 1);
-            return pc_key[h] == p ? pc_val[h] : J.phf[p];
-        };
-        auto term_s = [&](int t, float2 bh, int2 w, float& sr, float& si, int& cnt) {
-            if (bh.x == 0.f && bh.y == 0.f)
-                return;
-            const int2 sv = slot_v[t];
-            const int vx = (int)(short)(sv.x & 0xffff), vy = sv.x >> 16;
-            const int pu = wrap_idx(w.x - vx, w.y - vy, W, H), pv = sv.y;
-            if (!flag(pu) || !flag(pv))
-                return;
-            if (isnan(bh.x)) {
-                record_error(J.err, SMIP_DEV_ERR_OUT_OF_RANGE);
-                return;
-            }
-            const float2 ph = cmul(cmul(phase_of(pu), vtab[t]), make_float2(bh.x, -bh.y));
-            const float r = rsqrtf(ph.x * ph.x + ph.y * ph.y);
-            sr += ph.x * r;
-            si += ph.y * r;
-            ++cnt;
-        };
-        for (int q = 0; q < J.nvisits; ++q) {
-            load_plan(q + 1, c1); // its slots were loaded one visit ago
-            load_meta(q + 2, c2);
-            const int2 w = c0.w;
-            bool run = !(w.x < pmin0 || w.x > pmax0 || w.y < pmin1 || w.y > pmax1);
-            const int pw = run ? wrap_idx(w.x, w.y, W, H) : 0;
-            run = run && !flag(pw);
-            run = run && (abs(w.x) + abs(w.y) > 1);                                   // phasereco.h:84
-            run = run && !(w.x < umn0 || w.x > umx0 || w.y < umn1 || w.y > umx1);
-            // every visit's share lands (the summing warps do not know which
-            // visits run).  The slot is re-armed for visit q + kRing at once:
-            // its next share cannot land before progress passes q + kRing -
-            // kRecoLag, and an arrive here, before this visit's global stores,
-            // does not wait for them (an arrive is a release)
-            const int slot = q % kRing;
-            if (!__all_sync(0xffffffffu,
-                            wait_until([&] { return mbar_try_wait(&ring_bar[slot], (uint32_t)(q / kRing) & 1u); }) ? 1 : 0))
-                break;
-            if (lane == 0 && q + kRing < J.nvisits)
-                mbar_arrive_expect_tx(&ring_bar[slot], kShareBytes * nparts);
-            if (run) {
-                float sr = 0.f, si = 0.f;
-                int cnt = 0;
-                if (c0.rc >= 0) {
-                    if (c0.ta >= 0)
-                        term_s(c0.ta, c0.ba, w, sr, si, cnt);
-                    if (c0.tb >= 0)
-                        term_s(c0.tb, c0.bb, w, sr, si, cnt);
-                } else {
-                    sum_pairs(q, w, false, Local {}, phase_of, 0, nwords, sr, si, cnt);
-                }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    sr += __shfl_xor_sync(0xffffffffu, sr, o);
-                    si += __shfl_xor_sync(0xffffffffu, si, o);
-                    cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-                }
-                if (lane == 0) {
-                    // float-float: the non-recent share's parts in order, plus the recent one
-                    const float4 o4 = ring_s[slot][0];
-                    float rh = o4.x, rl = o4.y, ih = o4.z, il = o4.w;
-                    cnt += ring_n[slot][0];
-                    for (int pp = 1; pp < nparts; ++pp) {
-                        const float4 op = ring_s[slot][pp];
-                        ff_add(rh, rl, op.x, op.y);
-                        ff_add(ih, il, op.z, op.w);
-                        cnt += ring_n[slot][pp];
-                    }
-                    ff_add(rh, rl, sr, 0.f);
-                    ff_add(ih, il, si, 0.f);
-                    if (cnt > 0) {
-                        // FP32 phase for the chain; FP64 values are formed after the walk
-                        const float s2 = rh * rh + ih * ih;
-                        const float lim = 2.220446049250313e-16f * (float)cnt;
-                        float2 pf = make_float2(0.f, 0.f);
-                        if (s2 > lim * lim) {
-                            const float r = rsqrtf(s2);
-                            pf = make_float2(rh * r, ih * r);
-                        }
-                        J.phf[pw] = pf;
-                        J.sums[pw] = make_float4(rh, rl, ih, il);
-                        J.cnt[pw] = cnt;
-                        if (abs(w.x) <= De / 2 && abs(w.y) <= De / 2)
-                            vtab[(w.y + De / 2) * nside + w.x + De / 2] = pf;
-                        pc_val[pw & (kPhaseCache - 1)] = pf;
-                        pc_key[pw & (kPhaseCache - 1)] = pw;
-                        flagbits[pw >> 5] |= 1u << (pw & 31);
-                    }
-                }
-                __syncwarp();
-            }
-            // publish progress every 16 visits (a release store at cluster
-            // scope, which waits for this thread's stores to the phase map
-            // to reach every CTA; the lag leaves the slack)
-            if (((q & 15) == 15 || q + 1 == J.nvisits) && lane == 0)
-                dsmem_st_release(a_progress, q + 1);
-            __syncwarp();
-            c0 = c1;
-            c1 = c2;
-        }
-    } else {
-        // ------------------------------------------- non-recent shares
-        const int nsum = ncta > 1 ? (int)(ncta - 1) * (kRecoThreads / 32) : kRecoThreads / 32 - 1;
-        const int g = ncta > 1 ? (int)(rank - 1) * (kRecoThreads / 32) + warp : warp - 1;
-        const long long nitems = (long long)J.nvisits * nparts; // (visit, part), visits in order
-        for (long long it = (ncta > 1 && rank == 0) ? nitems : g; it < nitems; it += nsum) {
-            const int q = (int)(it / nparts), part = (int)(it - (long long)q * nparts);
-            if (!__all_sync(0xffffffffu, wait_until([&] { return dsmem_ld_acquire(a_progress) >= q - kRecoLag; }) ? 1 : 0))
-                break;
-            const int2 w = J.visits[q];
-            const int rc = J.rcount[q];
-            float sr = 0.f, si = 0.f;
-            int cnt = 0;
-            const bool inmap = !(w.x < pmin0 || w.x > pmax0 || w.y < pmin1 || w.y > pmax1);
-            if (rc >= 0 && inmap)
-                sum_pairs(q, w, true, Global {}, 0, (int)((long long)part * nwords / nparts),
-                          (int)((long long)(part + 1) * nwords / nparts), sr, si, cnt);
-            // float-float over the lanes, lane 0's order
-            float rh = sr, rl = 0.f, ih = si, il = 0.f;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const float a = __shfl_xor_sync(0xffffffffu, rh, o), b = __shfl_xor_sync(0xffffffffu, rl, o);
-                const float c = __shfl_xor_sync(0xffffffffu, ih, o), e = __shfl_xor_sync(0xffffffffu, il, o);
-                ff_add(rh, rl, a, b);
-                ff_add(ih, il, c, e);
-                cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-            }
-            if (lane == 0) {
-                const int slot = q % kRing;
-                const uint32_t bar = dsmem_addr(&ring_bar[slot], 0);
-                dsmem_st_async_f4(dsmem_addr(&ring_s[slot][part], 0), make_float4(rh, rl, ih, il), bar);
-                dsmem_st_async_i(dsmem_addr(&ring_n[slot][part], 0), cnt, bar);
-            }
-            __syncwarp();
-        }
-    }
-    cluster_sync_all(); // no CTA reads or writes rank 0's shared memory after this
-    if (rank != 0)
-        return;
-    // FP64 mean, consistency and phase of every point (phasereco.h:110-122),
-    // and the flag map
-    for (int p = threadIdx.x; p < nbits; p += blockDim.x) {
-        const unsigned f = (flagbits[p >> 5] >> (p & 31)) & 1u;
-        J.flags[p] = f;
-        if (!f)
-            continue;
-        const int n = J.cnt[p];
-        if (n < 0) { // seed
-            J.phases[p] = make_double2(1.0, J.phf[p].y);
-            J.cons[p] = 1.0;
-            continue;
-        }
-        const float4 s = J.sums[p];
-        const double mr = ((double)s.x + (double)s.y) / (double)n;
-        const double mi = ((double)s.z + (double)s.w) / (double)n;
-        const double ab = sqrt(mr * mr + mi * mi);
-        J.cons[p] = ab;
-        J.phases[p] = ab > 2.220446049250313080847263336181640625e-16 ? make_double2(mr / ab, mi / ab)
-                                                                      : make_double2(0.0, 0.0);
-    }
-}
-
-// The walk in one CTA per job (depths below kClusterDepth).  Warp 0 runs the visits in order: for visit q it
-// waits for the share of the non-recent pairs, adds the recent pairs (or all
-// pairs when the list overflowed), forms the phase and advances `progress`.
-// Warps 1..15 form the non-recent shares of visits q = warp-1 (mod 15), each
-// once progress >= q - kRecoLag, into a ring of kRing slots.  Every wait is
-// bounded; on a timeout the walk stops and the error is recorded.
-
-// CTA-scope acquire load / release store on shared memory: they order the
-// accesses after (before) them without waiting for this thread's other
-// outstanding loads, as a full fence would.
 __device__ __forceinline__ int ld_acquire_cta(const int* p)
 {
     int v;
     asm volatile("ld.acquire.cta.shared.b32 %0, [%1];" : "=r"(v) : "r"(smem_u32(p)) : "memory");
     return v;
 }
+// a plan row is read once: not kept in L1, which holds the phase map
+__device__ __forceinline__ float2 ld_stream(const float2* p)
+{
+    float2 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+}
 
-__global__ void __launch_bounds__(kRecoThreads, 1) phase_pipe_kernel(const RecoJob* __restrict__ jobs)
+static size_t walk_smem(int nslots) { return sizeof(float4) * (nslots + kRing * kRecentMax + kRing + 1) + sizeof(unsigned) * kRing * kRecentMax; }
+
+// CTAs per job: as few as keep the serial warp busy, because jobs that share
+// the GPU need the other SMs.  Cycles a visit with 1 / 2 / 4 CTAs: 583 / 493 /
+// 490 at depth 24, 708 / 595 / 475 at depth 32 (a lone CTA's summing warps have
+// three sub-partitions); at depth 48 seven summing CTAs keep up (461).
+static int walk_ctas(int De) { return De < 28 ? 2 : (De < kPartsDepth ? 4 : 8); }
+
+template <bool MULTI> // a cluster of CTAs per job, or one CTA
+__global__ void __launch_bounds__(kRecoThreads, 1) phase_walk_kernel(const RecoJob* __restrict__ jobs)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
-    __shared__ float4 ring_s[kRing];
-    __shared__ int ring_n[kRing];
-    __shared__ int ring_tag[kRing];
-    __shared__ int progress;
+    __shared__ float4 shr[kMaxParts + 1][kRing]; // share of the non-recent pairs: re hi, lo, im hi, lo; row kMaxParts: the parts' sum
+    __shared__ int shn[kMaxParts + 1][kRing];
+    __shared__ int tag_s[kMaxParts + 1][kRing];  // visit + 1 whose part has landed; row kMaxParts: all of it, gathered
+    __shared__ float4 ctl[kRing];            // phase the point already has (or NaN), kind of visit, kc | two sets << 8
+    __shared__ float4 res_s[kRing + 1];      // sums of the last visits, for the writer (+ a place for what nobody reads)
+    __shared__ __align__(8) uint64_t ring_bar[kRing];   // cluster: visit q's parts have landed in slot q mod kRing
+    __shared__ __align__(8) uint64_t done_bar[kGroups]; // the serial warp has finished kStep more visits
+    __shared__ int progress;   // visits whose phases are published (a copy in every CTA)
     __shared__ int abort_walk;
-    __shared__ int pc_key[kPhaseCache];   // serial warp: phases it set, by point
-    __shared__ float2 pc_val[kPhaseCache];
-    const RecoJob J = jobs[blockIdx.x];
-    const int W = J.W, H = J.H, De = J.De;
-    const int nbits = W * H;
-    const int nside = De + 1, nv = nside * nside, nwords = (nv + 31) / 32;
-    float2* vtab = reinterpret_cast<float2*>(smraw);                        // [nv] phases of the v disc
-    int2* slot_v = reinterpret_cast<int2*>(vtab + nv);                      // [nv] (vx | vy << 16, map index of v)
-    unsigned int* flagbits = reinterpret_cast<unsigned int*>(slot_v + nv);  // [W*H bits]
-    for (int i = threadIdx.x; i < (nbits + 31) / 32; i += blockDim.x)
-        flagbits[i] = 0u;
-    for (int i = threadIdx.x; i < nv; i += blockDim.x) {
-        vtab[i] = make_float2(0.f, 0.f);
-        const int vx = -De / 2 + i % nside, vy = -De / 2 + i / nside;
-        slot_v[i] = make_int2((int)(((unsigned)vx & 0xffffu) | ((unsigned)vy << 16)), wrap_idx(vx, vy, W, H));
+    const uint32_t rank = MULTI ? cluster_rank() : 0u, ncta = MULTI ? cluster_size() : 1u;
+    const RecoJob J = jobs[blockIdx.x / ncta];
+    const int W = J.W, H = J.H, De = J.De, e = De / 2;
+    const int nside = De + 1, nv = nside * nside, nwords = (nv + 31) / 32, nslots = nwords * 32;
+    const int nparts = share_parts(De, nwords), share_row = nparts > 1 ? kMaxParts : 0;
+    const int tag_row = MULTI ? kMaxParts : share_row; // what tells the serial warp that a visit has been posted
+    const int PW = W + De;
+    float4* vt = reinterpret_cast<float4*>(smraw); // [nslots] phase of v, map offset of v
+    float4* ent = vt + nslots;                     // [kRing][kRecentMax] phasor, the member outside the lag (rank 0)
+    float4* res_p = ent + kRing * kRecentMax;      // [kRing + 1] phases of the last visits, pairs of a point that got its phase
+    // where a recent pair's u and v lie, in units of 8 bytes from ent (a last
+    // phase's slot, or the posted member): u | v << 16, bits 14 and 30: the
+    // phase of the visit just before, bit 31: the phasor is out of range
+    unsigned* ecode = reinterpret_cast<unsigned*>(res_p + kRing + 1); // [kRing][kRecentMax]
+    const float nanf_ = __uint_as_float(kUnusable);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int t = threadIdx.x; t < nslots; t += blockDim.x) {
+        const int vx = -e + t % nside, vy = -e + t / nside;
+        float4 v = make_float4(nanf_, nanf_, __int_as_float(t < nv ? vy * PW + vx : 0), 0.f);
+        if (t < nv && abs(vx) + abs(vy) <= 1) { // seeds (phasereco.h:42-54)
+            v.x = 1.f;
+            v.y = vx < 0 || vy < 0 ? -0.f : 0.f;
+            if (rank == 0) {
+                const int p = wrap_idx(vx, vy, W, H);
+                J.pmap[(vy + (H >> 1) + e) * PW + vx + (W >> 1) + e] = make_float2(v.x, v.y);
+                J.sums[p] = make_float4(0.f, 0.f, 0.f, 0.f);
+                J.cnt[p] = -1;
+            }
+        }
+        vt[t] = v;
     }
-    for (int i = threadIdx.x; i < kRing; i += blockDim.x)
-        ring_tag[i] = -1;
+    for (int i = threadIdx.x; i < (kMaxParts + 1) * kRing; i += blockDim.x)
+        (&tag_s[0][0])[i] = 0;
+    // a slot is read before its first pairs are posted (a visit with nothing
+    // to sum posts none): its codes must be places within ent at all times
+    for (int i = threadIdx.x; i < kRing * kRecentMax; i += blockDim.x)
+        ecode[i] = 0u;
     if (threadIdx.x == 0) {
         progress = 0;
         abort_walk = 0;
+        for (int i = 0; i < kRing; ++i)
+            mbar_init(&ring_bar[i], nparts); // an arrival per part
+        for (int i = 0; i < kGroups; ++i)
+            mbar_init(&done_bar[i], 1);
+        fence_mbar_init();
     }
-    __syncthreads();
-    if (threadIdx.x < 5) { // seeds (phasereco.h:42-54); all inside the v disc
-        const int sx[5] = { 0, 1, 0, -1, 0 }, sy[5] = { 0, 0, 1, 0, -1 };
-        const int p = wrap_idx(sx[threadIdx.x], sy[threadIdx.x], W, H);
-        const float im = threadIdx.x < 3 ? 0.f : -0.f;
-        J.phf[p] = make_float2(1.f, im);
-        J.sums[p] = make_float4(0.f, 0.f, 0.f, 0.f);
-        J.cnt[p] = -1;
-        vtab[(sy[threadIdx.x] + De / 2) * nside + sx[threadIdx.x] + De / 2] = make_float2(1.f, im);
-        atomicOr(&flagbits[p >> 5], 1u << (p & 31));
-    }
-    __syncthreads();
-    const int pmin0 = -(W >> 1), pmin1 = -(H >> 1);
-    const int pmax0 = -W / 2 + W - 1, pmax1 = -H / 2 + H - 1;
-    const int szW = (W / 2) * 2 + 1, szH = (H / 2) * 2 + 1;
-    const int umn0 = -(szW / 2), umx0 = szW - szW / 2 - 1, umn1 = -(szH / 2), umx1 = szH - szH / 2 - 1;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    volatile int* vabort = &abort_walk;
+    __threadfence(); // the seeds in the map
+    if constexpr (MULTI)
+        cluster_sync_all();
+    else
+        __syncthreads();
 
-    auto flag = [&](int p) { return ((flagbits[p >> 5] >> (p & 31)) & 1u) != 0u; };
-    // bounded wait on a shared-memory condition; false on a timeout (then the walk stops)
-    auto wait_until = [&](auto cond) {
+    auto aborted = [&]() {
+        if constexpr (MULTI)
+            return dsmem_ld_relaxed(dsmem_addr(&abort_walk, 0)) != 0;
+        else
+            return *reinterpret_cast<volatile int*>(&abort_walk) != 0;
+    };
+    auto give_up = [&]() {
+        if constexpr (MULTI)
+            dsmem_st_relaxed(dsmem_addr(&abort_walk, 0), 1);
+        else
+            *reinterpret_cast<volatile int*>(&abort_walk) = 1;
+    };
+    // bounded wait on a condition; false on a timeout or when another warp
+    // gave up (then the walk stops)
+    auto wait_until = [&](auto cond, unsigned sleep) {
         if (cond())
             return true;
         const unsigned long long t0 = globaltimer_ns();
         for (;;) {
-            for (int i = 0; i < 64; ++i)
+            for (int i = 0; i < 64; ++i) {
                 if (cond())
                     return true;
-            if (*vabort)
+                if (sleep)
+                    __nanosleep(sleep);
+            }
+            if (aborted())
                 return false;
             if (globaltimer_ns() - t0 > kRecoWaitNs) {
                 record_error(J.err, SMIP_DEV_ERR_TIMEOUT);
-                *vabort = 1;
+                give_up();
                 return false;
             }
         }
     };
-
-    // Pairs of visit q, eight slots per lane at a time, so that the plan,
-    // flag and phase gathers overlap; skip_recent leaves the recent pairs
-    // out (the serial warp takes them); phase reads the phase map.
-    auto sum_pairs = [&](int q, int2 w, bool skip_recent, auto phase, float& sr, float& si, int& cnt) {
-        constexpr int kB = 8;
-        const unsigned* rb = J.rbits + (long long)q * nwords;
-        const float2* prow = J.plan + (long long)q * nv;
-        for (int i0 = 0; i0 < nwords; i0 += kB) {
-            float2 bh[kB], ph[kB];
-            int tt[kB];
-            bool use[kB];
-#pragma unroll
-            for (int k = 0; k < kB; ++k) {
-                const int t = lane + 32 * (i0 + k);
-                tt[k] = t;
-                use[k] = i0 + k < nwords && t < nv;
-                // slot t's bit is bit `lane` of word i0 + k
-                if (skip_recent)
-                    use[k] = use[k] && !((rb[i0 + k] >> lane) & 1u);
-                bh[k] = use[k] ? prow[t] : make_float2(0.f, 0.f);
-                if (use[k]) { // flags and the phase gather do not wait for the plan
-                    const int2 sv = slot_v[t];
-                    const int vx = (int)(short)(sv.x & 0xffff), vy = sv.x >> 16;
-                    const int ux = w.x - vx, uy = w.y - vy;
-                    const bool inu = !(ux < pmin0 || ux > pmax0 || uy < pmin1 || uy > pmax1);
-                    const int pu = inu ? wrap_idx(ux, uy, W, H) : 0, pv = sv.y;
-                    use[k] = inu && flag(pu) && flag(pv);
-                    ph[k] = use[k] ? phase(pu) : make_float2(0.f, 0.f);
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < kB; ++k) {
-                if (!use[k] || (bh[k].x == 0.f && bh[k].y == 0.f)) // the plan's zero: never contributes
-                    continue;
-                if (isnan(bh[k].x)) {
-                    record_error(J.err, SMIP_DEV_ERR_OUT_OF_RANGE);
-                    continue;
-                }
-                const float2 p = cmul(cmul(ph[k], vtab[tt[k]]), make_float2(bh[k].x, -bh[k].y));
-                const float r = rsqrtf(p.x * p.x + p.y * p.y);
-                sr += p.x * r;
-                si += p.y * r;
-                ++cnt;
-            }
-        }
+    const bool oor_any = *J.oor != 0;
+    auto check_oor = [&](bool is_oor, float2 U, float2 V) { // get_element would throw in a pair that is used
+        if (is_oor && !isnan(U.x) && !isnan(V.x))
+            record_error(J.err, SMIP_DEV_ERR_OUT_OF_RANGE);
     };
 
-    if (warp == 0) {
+    const bool on_rank0 = !MULTI || rank == 0;
+    if (on_rank0 && warp == 0) {
         // ------------------------------------------------ serial warp
-        // Visit data that does not depend on the walk is loaded ahead: the
-        // visit, its recent-pair count and slots two visits ahead, their plan
-        // phasors one visit ahead.  Phases the walk just set come from a
-        // shared-memory cache keyed by point (a miss reads the phase map).
-        for (int i = lane; i < kPhaseCache; i += 32)
-            pc_key[i] = -1;
-        __syncwarp();
-        struct Ahead {
-            int2 w;
-            int rc, ta, tb;
-            float2 ba, bb;
+        struct Vis { // a visit as posted
+            float2 bh; // phasor
+            unsigned c; // where its members lie
+            float4 k;  // ctl
         };
-        // the list slots are loaded without waiting for the count (a visit's
-        // kRecentMax entries are always allocated) and masked one visit later
-        auto load_meta = [&](int q, Ahead& a) {
-            if (q >= J.nvisits)
-                return;
-            a.w = J.visits[q];
-            a.rc = J.rcount[q];
-            const unsigned short* rl = J.rlist + (long long)q * kRecentMax;
-            a.ta = rl[lane];
-            a.tb = rl[lane + 32];
+        const float2* mem = reinterpret_cast<const float2*>(ent);
+        auto load_vis = [&](int q, Vis& v) {
+            const int s = q & (kRing - 1);
+            v.bh = mem[2 * (s * kRecentMax + lane)];
+            v.c = ecode[s * kRecentMax + lane];
+            v.k = ctl[s];
         };
-        auto load_plan = [&](int q, Ahead& a) {
-            if (q >= J.nvisits)
-                return;
-            a.ta = lane < a.rc ? a.ta : -1;
-            a.tb = lane + 32 < a.rc ? a.tb : -1;
-            const float2* prow = J.plan + (long long)q * nv;
-            a.ba = a.ta >= 0 ? prow[a.ta] : make_float2(0.f, 0.f);
-            a.bb = a.tb >= 0 ? prow[a.tb] : make_float2(0.f, 0.f);
+        auto members = [&](unsigned c, float2& U, float2& V) {
+            U = mem[c & 0x3fffu];
+            V = mem[(c >> 16) & 0x3fffu];
         };
-        Ahead c0 {}, c1 {}, c2 {};
-        load_meta(0, c0);
-        load_plan(0, c0);
-        load_meta(1, c1);
-        auto phase_of = [&](int p) {
-            const int h = p & (kPhaseCache - 1);
-            return pc_key[h] == p ? pc_val[h] : J.phf[p];
+        auto term = [&](float2 U, float2 V, float2 bh, float2& p, float& r) {
+            p = pair_product(U, V, bh.x, bh.y);
+            const float n2 = norm2(p);
+            r = rsqrt_ftz(n2);
+            return !isnan(n2);
         };
-        auto term_s = [&](int t, float2 bh, int2 w, float& sr, float& si, int& cnt) {
-            if (bh.x == 0.f && bh.y == 0.f)
-                return;
-            const int2 sv = slot_v[t];
-            const int vx = (int)(short)(sv.x & 0xffff), vy = sv.x >> 16;
-            const int pu = wrap_idx(w.x - vx, w.y - vy, W, H), pv = sv.y;
-            if (!flag(pu) || !flag(pv))
-                return;
-            if (isnan(bh.x)) {
-                record_error(J.err, SMIP_DEV_ERR_OUT_OF_RANGE);
-                return;
-            }
-            const float2 ph = cmul(cmul(phase_of(pu), vtab[t]), make_float2(bh.x, -bh.y));
-            const float r = rsqrtf(ph.x * ph.x + ph.y * ph.y);
-            sr += ph.x * r;
-            si += ph.y * r;
-            ++cnt;
+        // a point's phase from its float-float sum and number of pairs; FP64
+        // values are formed after the walk.  A sum above the limit has a
+        // normal square.
+        auto phase_from = [&](float4 sum, int cnt) {
+            const float s2 = norm2(make_float2(sum.x, sum.z));
+            const float lim = 2.220446049250313e-16f * (float)cnt;
+            const float r = rsqrt_ftz(s2);
+            float2 pf = s2 > lim * lim ? make_float2(sum.x * r, sum.z * r) : make_float2(0.f, 0.f);
+            pf.x = cnt > 0 ? pf.x : nanf_; // no pair: no phase
+            pf.y = cnt > 0 ? pf.y : nanf_;
+            return pf;
         };
-        for (int q = 0; q < J.nvisits; ++q) {
-            load_plan(q + 1, c1); // its slots were loaded one visit ago
-            load_meta(q + 2, c2);
-            const int2 w = c0.w;
-            bool run = !(w.x < pmin0 || w.x > pmax0 || w.y < pmin1 || w.y > pmax1);
-            const int pw = run ? wrap_idx(w.x, w.y, W, H) : 0;
-            run = run && !flag(pw);
-            run = run && (abs(w.x) + abs(w.y) > 1);                                   // phasereco.h:84
-            run = run && !(w.x < umn0 || w.x > umx0 || w.y < umn1 || w.y > umx1);
-            if (run) {
-                const int slot = q % kRing;
-                if (!__all_sync(0xffffffffu, wait_until([&] { return ld_acquire_cta(&ring_tag[slot]) == q; }) ? 1 : 0))
-                    break;
-                float sr = 0.f, si = 0.f;
-                int cnt = 0;
-                if (c0.rc >= 0) {
-                    if (c0.ta >= 0)
-                        term_s(c0.ta, c0.ba, w, sr, si, cnt);
-                    if (c0.tb >= 0)
-                        term_s(c0.tb, c0.bb, w, sr, si, cnt);
-                } else {
-                    sum_pairs(q, w, false, phase_of, sr, si, cnt);
+        // visits [q, q + kStep) (or up to the last) are ready: relaxed polls and
+        // one fence of this CTA's scope, which costs nothing (a fence of the
+        // cluster's takes 300 cycles: the gathering warps do those)
+        auto ready = [&](int q) {
+            const int v = q + (lane & (kStep - 1)) < J.nvisits ? q + (lane & (kStep - 1)) : J.nvisits - 1;
+            const volatile int* tag = &tag_s[tag_row][v & (kRing - 1)];
+            unsigned long long t0 = 0;
+            for (int n = 1;; ++n) {
+                if (__all_sync(0xffffffffu, *tag == v + 1)) {
+                    __threadfence_block();
+                    return true;
                 }
+                if (n & 63)
+                    continue;
+                const unsigned long long now = globaltimer_ns();
+                t0 = t0 ? t0 : now;
+                const bool late = now - t0 > kRecoWaitNs;
+                if (late && lane == 0) {
+                    record_error(J.err, SMIP_DEV_ERR_TIMEOUT);
+                    give_up();
+                }
+                if (__any_sync(0xffffffffu, late || aborted()))
+                    return false;
+            }
+        };
+        const int nqs = (J.nvisits + kStep - 1) / kStep * kStep; // the writer leaves out what lies past the last visit
+        Vis v0, v1, v2; // visits q, q + 1, q + 2
+        // what is known of visit q before the phase of visit q - 1
+        float2 eU, eV;      // members (lane 0: one of them is that phase)
+        float sR[5], sI[5]; // the sibling sums of the butterfly's levels
+        int ecnt;           // pairs but lane 0's, and the share's
+        float4 esum;        // share of the non-recent pairs
+        auto early = [&](int q, const Vis& v) {
+            esum = shr[share_row][q & (kRing - 1)];
+            ecnt = shn[share_row][q & (kRing - 1)];
+            float2 p;
+            float r;
+            const bool ok = term(eU, eV, v.bh, p, r);
+            float x = ok ? fmaf(p.x, r, 0.f) : 0.f, y = ok ? fmaf(p.y, r, 0.f) : 0.f;
+            ecnt += __popc(__ballot_sync(0xffffffffu, ok) & ~1u);
+#pragma unroll
+            for (int l = 0; l < 5; ++l) {
+                sR[l] = __shfl_xor_sync(0xffffffffu, x, 16 >> l);
+                sI[l] = __shfl_xor_sync(0xffffffffu, y, 16 >> l);
+                x = __fadd_rn(x, sR[l]);
+                y = __fadd_rn(y, sI[l]);
+            }
+        };
+        float2 last = make_float2(nanf_, nanf_);
+        // every lane stores a visit's result, lane 0 (whose result it is) to
+        // its slot, the others to a slot that nobody reads
+        const int smul = lane == 0 ? 1 : 0, sadd = lane == 0 ? 0 : kRing;
+        auto store = [&](int q, float4 sum, int cnt) {
+            const int s = (q & (kRing - 1)) * smul + sadd;
+            res_p[s] = make_float4(last.x, last.y, __int_as_float(cnt), 0.f);
+            res_s[s] = sum;
+        };
+        bool go = ready(0) && ready(2);
+        if (go) {
+            load_vis(0, v0);
+            load_vis(1, v1);
+            members(v0.c, eU, eV);
+            early(0, v0);
+        }
+        for (int q = 0; go && q < nqs;) {
+            if (__float_as_int(v0.k.z) != kWide) {
+                // The loop's body is one block without branches, for the fast
+                // visits and those with nothing to do, so that the chain of
+                // visit q (lane 0) and the early part of visit q + 1 overlap.
+                do {
+                    load_vis(q + 2, v2); // used one visit later
+                    const int kind = __float_as_int(v0.k.z);
+                    float2 nU, nV;
+                    members(v1.c, nU, nV);
+                    const bool lu = v0.c & 0x4000u, lv = v0.c & 0x40000000u;
+                    const float2 U = make_float2(lu ? last.x : eU.x, lu ? last.y : eU.y);
+                    const float2 V = make_float2(lv ? last.x : eV.x, lv ? last.y : eV.y);
+                    float2 p;
+                    float r;
+                    const bool ok = term(U, V, v0.bh, p, r);
+                    float x = ok ? fmaf(p.x, r, 0.f) : 0.f, y = ok ? fmaf(p.y, r, 0.f) : 0.f;
+    #pragma unroll
+                    for (int l = 0; l < 5; ++l) {
+                        x = __fadd_rn(x, sR[l]);
+                        y = __fadd_rn(y, sI[l]);
+                    }
+                    int cnt = ecnt + (ok ? 1 : 0);
+                    float4 sum = esum;
+                    ff_add(sum.x, sum.y, x, 0.f);
+                    ff_add(sum.z, sum.w, y, 0.f);
+                    last = phase_from(sum, cnt);
+                    cnt = kind == kFast ? cnt : 0;
+                    last.x = kind == kFast ? last.x : v0.k.x;
+                    last.y = kind == kFast ? last.y : v0.k.y;
+                    eU = nU;
+                    eV = nV;
+                    early(q + 1, v1);
+                    store(q, sum, cnt);
+                    __syncwarp();
+                    v0 = v1;
+                    v1 = v2;
+                    ++q;
+                } while (((q & (kStep - 1)) != 0) & (__float_as_int(v0.k.z) != kWide));
+            } else { // all terms now: the phases up to the last lie in their slots
+                load_vis(q + 2, v2);
+                const int s = q & (kRing - 1), kc = __float_as_int(v0.k.w) & 63;
+                const bool two = (__float_as_int(v0.k.w) >> 8) != 0;
+                float2 Ua, Va, Ub, Vb, pa, pb;
+                float ra, rb;
+                members(v0.c, Ua, Va);
+                const unsigned cb = ecode[s * kRecentMax + 32 + lane];
+                const float2 bb = mem[2 * (s * kRecentMax + 32 + lane)];
+                members(cb, Ub, Vb);
+                const float4 own = res_p[(q - kc) & (kRing - 1)];
+                float4 sum = shr[share_row][s];
+                int cnt = shn[share_row][s];
+                const bool oka = term(Ua, Va, v0.bh, pa, ra);
+                const bool okb = term(Ub, Vb, bb, pb, rb) && two;
+                float sr = oka ? fmaf(pa.x, ra, 0.f) : 0.f, si = oka ? fmaf(pa.y, ra, 0.f) : 0.f;
+                sr = okb ? fmaf(pb.x, rb, sr) : sr;
+                si = okb ? fmaf(pb.y, rb, si) : si;
+                cnt += __popc(__ballot_sync(0xffffffffu, oka)) + __popc(__ballot_sync(0xffffffffu, okb));
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) {
-                    sr += __shfl_xor_sync(0xffffffffu, sr, o);
-                    si += __shfl_xor_sync(0xffffffffu, si, o);
-                    cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+                    sr = __fadd_rn(sr, __shfl_xor_sync(0xffffffffu, sr, o));
+                    si = __fadd_rn(si, __shfl_xor_sync(0xffffffffu, si, o));
                 }
-                if (lane == 0) {
-                    // float-float: the non-recent share plus the recent one
-                    const float4 o4 = ring_s[slot];
-                    float rh = o4.x, rl = o4.y, ih = o4.z, il = o4.w;
-                    ff_add(rh, rl, sr, 0.f);
-                    ff_add(ih, il, si, 0.f);
-                    cnt += ring_n[slot];
-                    if (cnt > 0) {
-                        // FP32 phase for the chain; FP64 values are formed after the walk
-                        const float s2 = rh * rh + ih * ih;
-                        const float lim = 2.220446049250313e-16f * (float)cnt;
-                        float2 pf = make_float2(0.f, 0.f);
-                        if (s2 > lim * lim) {
-                            const float r = rsqrtf(s2);
-                            pf = make_float2(rh * r, ih * r);
+                ff_add(sum.x, sum.y, sr, 0.f);
+                ff_add(sum.z, sum.w, si, 0.f);
+                last = phase_from(sum, cnt);
+                if (kc && !isnan(own.x)) { // its point, visited within the lag, has its phase
+                    last = make_float2(own.x, own.y);
+                    cnt = 0;
+                } else if (oor_any && q < J.nvisits) {
+                    check_oor(v0.c >> 31, Ua, Va);
+                    check_oor(two && (cb >> 31), Ub, Vb);
+                }
+                members(v1.c, eU, eV);
+                early(q + 1, v1);
+                store(q, sum, cnt);
+                __syncwarp();
+                v0 = v1;
+                v1 = v2;
+                ++q;
+            }
+            if ((q & (kStep - 1)) == 0) { // tell the writer, look ahead
+                if (lane == 0)
+                    mbar_arrive(&done_bar[(q / kStep - 1) & (kGroups - 1)]);
+                go = ready(q + 2);
+            }
+        }
+    } else if (on_rank0 && warp == (MULTI ? 5 : 4)) {
+        // ------------------------------------------------------ writer
+        const int ngroups = (J.nvisits + kStep - 1) / kStep;
+        for (int g = 0; g < ngroups;) {
+            // groups of kStep visits, as many as are done (up to 32 visits)
+            auto is_done = [&](int h) { return mbar_test_wait(&done_bar[h & (kGroups - 1)], (uint32_t)(h / kGroups) & 1u); };
+            if (!__all_sync(0xffffffffu, wait_until([&] { return is_done(g); }, 20u) ? 1 : 0))
+                break;
+            const unsigned m8 = __ballot_sync(0xffffffffu, lane < 32 / kStep && g + lane < ngroups && is_done(g + lane)) | 1u;
+            const int n = __ffs(~m8) - 1;
+            const int q = kStep * g + lane, s = q & (kRing - 1);
+            if (lane < kStep * n && q < J.nvisits) {
+                const float4 rp = res_p[s];
+                const int cnt = __float_as_int(rp.z);
+                if (cnt > 0) { // a point got its phase
+                    const int4 m = J.meta[q];
+                    const float2 pf = make_float2(rp.x, rp.y);
+                    J.pmap[m.x] = pf;
+                    J.sums[m.y] = res_s[s];
+                    J.cnt[m.y] = cnt;
+                    if (m.w >= 0) {
+                        if constexpr (MULTI) {
+                            for (uint32_t c = 0; c < ncta; ++c)
+                                dsmem_st_f2(dsmem_addr(&vt[m.w], c), pf);
+                        } else {
+                            *reinterpret_cast<float2*>(&vt[m.w]) = pf;
                         }
-                        J.phf[pw] = pf;
-                        J.sums[pw] = make_float4(rh, rl, ih, il);
-                        J.cnt[pw] = cnt;
-                        if (abs(w.x) <= De / 2 && abs(w.y) <= De / 2)
-                            vtab[(w.y + De / 2) * nside + w.x + De / 2] = pf;
-                        pc_val[pw & (kPhaseCache - 1)] = pf;
-                        pc_key[pw & (kPhaseCache - 1)] = pw;
-                        flagbits[pw >> 5] |= 1u << (pw & 31);
                     }
                 }
-                __syncwarp();
             }
-            // publish progress every 8 visits (a release store; the lag leaves
-            // the slack)
-            if (((q & 7) == 7 || q + 1 == J.nvisits) && lane == 0)
-                st_release_cta(&progress, q + 1);
+            g += n;
             __syncwarp();
-            c0 = c1;
-            c1 = c2;
+            // release: the stores above come before it for whoever acquires it
+            if constexpr (MULTI) {
+                if (lane < (int)ncta)
+                    dsmem_st_release(dsmem_addr(&progress, lane), kStep * g);
+            } else {
+                if (lane == 0)
+                    st_release_cta(&progress, kStep * g);
+            }
+            __syncwarp();
         }
-    } else {
-        // ------------------------------------------- non-recent shares
-        for (int q = warp - 1; q < J.nvisits; q += kRecoThreads / 32 - 1) {
-            if (!__all_sync(0xffffffffu, wait_until([&] { return ld_acquire_cta(&progress) >= q - kRecoLag; }) ? 1 : 0))
+    } else if (on_rank0 && tag_row == kMaxParts && (MULTI ? warp < 4 || warp == 6 : warp == 8 || warp == 12)) {
+        // gathering warps: a visit's parts, in part order, and the other CTAs'
+        // data on to the serial warp
+        const int c = MULTI ? (warp == 6 ? 3 : warp - 1) : warp / 4 - 2, ncomb = MULTI ? 4 : 2;
+        for (int q = c; q < J.nvisits; q += ncomb) {
+            const int s = q & (kRing - 1);
+            const volatile int* tag = &tag_s[lane < nparts ? lane : 0][s];
+            if (!__all_sync(0xffffffffu, wait_until([&] {
+                                return MULTI ? mbar_try_wait_cluster(&ring_bar[s], (uint32_t)(q / kRing) & 1u) : *tag == q + 1;
+                            }, MULTI ? 0u : 20u) ? 1 : 0))
                 break;
-            const int2 w = J.visits[q];
-            const int rc = J.rcount[q];
+            __threadfence_block();
+            if (nparts > 1) {
+                float4 sum = shr[0][s];
+                int n = shn[0][s];
+                for (int pp = 1; pp < nparts; ++pp) {
+                    const float4 op = shr[pp][s];
+                    ff_add(sum.x, sum.y, op.x, op.y);
+                    ff_add(sum.z, sum.w, op.z, op.w);
+                    n += shn[pp][s];
+                }
+                if (lane == 0) {
+                    shr[kMaxParts][s] = sum;
+                    shn[kMaxParts][s] = n;
+                }
+            }
+            __syncwarp();
+            if (lane == 0)
+                st_release_cta(&tag_s[kMaxParts][s], q + 1);
+        }
+    } else if (MULTI ? rank != 0 : (warp & 3) != 0) {
+        // ------------------------------------------- non-recent shares
+        const int nsum = MULTI ? (int)(ncta - 1) * (kRecoThreads / 32) : kRecoThreads / 32 * 3 / 4;
+        const int g = MULTI ? (int)(rank - 1) * (kRecoThreads / 32) + warp : (warp >> 2) * 3 + (warp & 3) - 1;
+        const long long nitems = (long long)J.nvisits * nparts; // (visit, part), visits in order
+        // A part's words in nbat batches of nbw or nbw - 1: the pair slots per
+        // lane in flight, as many as the registers hold (18 spilled).
+        constexpr int kB = 10;
+        const int longest = (nwords + nparts - 1) / nparts;
+        const int nbat = (longest + kB - 1) / kB, nbw = (longest + nbat - 1) / nbat;
+        for (long long it = g; it < nitems; it += nsum) {
+            const int q = (int)(it / nparts), part = (int)(it - (long long)q * nparts);
+            const int wb = part * nwords / nparts, we = (part + 1) * nwords / nparts;
+            const int4 m = J.meta[q];
+            const float2* prow = J.plan + (long long)q * nslots + lane;
+            uint4 ra = make_uint4(kUnusable, kUnusable, 0u, 0u), rb = ra;
+            const int rc = m.z & 255, kc = (m.z >> 8) & 63;
+            const bool run = (m.z >> 17) & 1;
+            if (part == 0 && run) {
+                ra = J.rec[(long long)q * kRecentMax + lane];
+                if (rc > 32)
+                    rb = J.rec[(long long)q * kRecentMax + 32 + lane];
+            }
+            if (lane == 0 && it + nsum < nitems) { // the next item's plan row on its way into L2
+                const long long nx = it + nsum;
+                const int nq = (int)(nx / nparts), np = (int)(nx - (long long)nq * nparts);
+                const int b = np * nwords / nparts, l = (np + 1) * nwords / nparts - b;
+                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(J.plan + (long long)nq * nslots + 32 * b),
+                             "r"(l * 32 * (int)sizeof(float2))
+                             : "memory");
+            }
+            if (!__all_sync(0xffffffffu, wait_until([&] {
+                                const int pr = MULTI ? dsmem_ld_acquire(dsmem_addr(&progress, rank)) : ld_acquire_cta(&progress);
+                                return pr >= q - kRecoLag;
+                            }, 20u) ? 1 : 0))
+                break;
+            // the map: other SMs write it in a cluster (read from L2), this SM in a lone CTA
+            auto map_at = [&](long long i) { return MULTI ? __ldcg(J.pmap + i) : *(J.pmap + i); };
+            float2 cur = make_float2(nanf_, nanf_);
+            if (m.x >= 0)
+                cur = map_at(m.x);
+            // a point outside the map, a seed, or one that has its phase: nothing to sum
+            const bool skip = !run || (kc == 0 && !isnan(cur.x));
+            const int s = q & (kRing - 1);
+            const uint32_t bar = MULTI ? dsmem_addr(&ring_bar[s], 0) : 0u;
+            auto put4 = [&](float4* p, float4 v) {
+                if constexpr (MULTI)
+                    dsmem_st_async_f4(dsmem_addr(p, 0), v, bar);
+                else
+                    *p = v;
+            };
+            auto put1 = [&](int* p, int v) {
+                if constexpr (MULTI)
+                    dsmem_st_async_i(dsmem_addr(p, 0), v, bar);
+                else
+                    *p = v;
+            };
+            if (MULTI && lane == 0) // share and count; ctl; the recent pairs
+                dsmem_mbar_arrive_expect_tx(bar, 20u + (part == 0 ? 16u + (skip ? 0u : rc > 32 ? 1280u : 640u) : 0u));
+            if (part == 0) {
+                // the recent pairs, with their members outside the lag: their phases are final
+                auto post = [&](int at, uint4 r) {
+                    const int t = r.z & 0x1fff, ku = (r.z >> 13) & 63, kv = (r.z >> 19) & 63;
+                    const float4 sv = vt[t];
+                    float2 x = make_float2(sv.x, sv.y); // v, unless u is the one outside the lag
+                    if (!ku)
+                        x = map_at((long long)m.x - __float_as_int(sv.z));
+                    put4(&ent[s * kRecentMax + at], make_float4(__uint_as_float(r.x), __uint_as_float(r.y), x.x, x.y));
+                    const int own = 2 * (s * kRecentMax + at) + 1, lst = 2 * kRing * kRecentMax;
+                    const unsigned cu = ku ? lst + 2 * ((q - ku) & (kRing - 1)) : own;
+                    const unsigned cv = kv ? lst + 2 * ((q - kv) & (kRing - 1)) : own;
+                    put1(reinterpret_cast<int*>(&ecode[s * kRecentMax + at]),
+                         (int)(cu | cv << 16 | (ku == 1 ? 0x4000u : 0u) | (kv == 1 ? 0x40000000u : 0u)
+                               | ((r.z >> 25) & 1u) << 31));
+                };
+                if (!skip) {
+                    post(lane, ra);
+                    if (rc > 32)
+                        post(lane + 32, rb);
+                }
+                if (lane == 0) {
+                    const int kind = skip ? kSkip : ((m.z >> 16) & 1 && !oor_any ? kFast : kWide);
+                    put4(&ctl[s], make_float4(cur.x, cur.y, __int_as_float(kind),
+                                              __int_as_float(kc | (rc > 32 ? 1 << 8 : 0))));
+                }
+            }
             float sr = 0.f, si = 0.f;
             int cnt = 0;
-            const bool inmap = !(w.x < pmin0 || w.x > pmax0 || w.y < pmin1 || w.y > pmax1);
-            if (rc >= 0 && inmap)
-                sum_pairs(q, w, true, [&](int pu) { return J.phf[pu]; }, sr, si, cnt);
+            if (!skip) {
+                const float2* mb = J.pmap + m.x;
+                // NB: words of the longest batch, the others one less (GUARD:
+                // any number).  OOR: look for out-of-range elements too.
+                auto sum_pairs = [&](auto nbw, auto guard, auto oor) {
+                    constexpr int NB = decltype(nbw)::value;
+                    constexpr bool GUARD = decltype(guard)::value, OOR = decltype(oor)::value;
+                    for (int b = 0; b < nbat; ++b) {
+                        const int i0 = wb + b * (we - wb) / nbat, n = wb + (b + 1) * (we - wb) / nbat - i0;
+                        const float2* pw = prow + 32 * i0;
+                        const float4* vw = vt + 32 * i0 + lane;
+                        float2 bh[NB], u[NB], v[NB];
+#pragma unroll
+                        for (int k = 0; k < NB; ++k) {
+                            const int i = (GUARD || k == NB - 1) && k >= n ? 0 : 32 * k;
+                            const float4 sl = vw[i];
+                            v[k] = make_float2(sl.x, sl.y);
+                            bh[k] = ld_stream(pw + i);
+                            const float2* up = mb - __float_as_int(sl.z);
+                            u[k] = MULTI ? __ldcg(up) : *up;
+                        }
+#pragma unroll
+                        for (int k = 0; k < NB; ++k) {
+                            const bool in = !((GUARD || k == NB - 1) && k >= n);
+                            const float2 p = pair_product(u[k], v[k], bh[k].x, bh[k].y);
+                            const float n2 = norm2(p);
+                            const float r = rsqrt_ftz(n2);
+                            if (in && !isnan(n2)) {
+                                sr = fmaf(p.x, r, sr);
+                                si = fmaf(p.y, r, si);
+                                ++cnt;
+                            }
+                            if constexpr (OOR)
+                                check_oor(in && __float_as_uint(bh[k].x) == kOorBits, u[k], v[k]);
+                        }
+                    }
+                };
+                using Yes = std::true_type;
+                using No = std::false_type;
+                if (oor_any)
+                    sum_pairs(std::integral_constant<int, kB> {}, Yes {}, Yes {});
+                else if (nbw == 10)
+                    sum_pairs(std::integral_constant<int, 10> {}, No {}, No {});
+                else if (nbw == 9)
+                    sum_pairs(std::integral_constant<int, 9> {}, No {}, No {});
+                else if (nbw == 8)
+                    sum_pairs(std::integral_constant<int, 8> {}, No {}, No {});
+                else if (nbw == 7)
+                    sum_pairs(std::integral_constant<int, 7> {}, No {}, No {});
+                else
+                    sum_pairs(std::integral_constant<int, 6> {}, Yes {}, No {});
+            }
             // float-float over the lanes, lane 0's order
             float rh = sr, rl = 0.f, ih = si, il = 0.f;
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
                 const float a = __shfl_xor_sync(0xffffffffu, rh, o), b = __shfl_xor_sync(0xffffffffu, rl, o);
-                const float c = __shfl_xor_sync(0xffffffffu, ih, o), e = __shfl_xor_sync(0xffffffffu, il, o);
+                const float c = __shfl_xor_sync(0xffffffffu, ih, o), f = __shfl_xor_sync(0xffffffffu, il, o);
                 ff_add(rh, rl, a, b);
-                ff_add(ih, il, c, e);
-                cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+                ff_add(ih, il, c, f);
             }
+            cnt = __reduce_add_sync(0xffffffffu, cnt);
             if (lane == 0) {
-                const int slot = q % kRing;
-                ring_s[slot] = make_float4(rh, rl, ih, il);
-                ring_n[slot] = cnt;
-                st_release_cta(&ring_tag[slot], q);
+                put4(&shr[part][s], make_float4(rh, rl, ih, il));
+                put1(&shn[part][s], cnt);
             }
-            __syncwarp();
+            if constexpr (!MULTI) {
+                __syncwarp();
+                if (lane == 0)
+                    st_release_cta(&tag_s[part][s], q + 1);
+            }
         }
     }
-    __syncthreads();
-    // FP64 mean, consistency and phase of every point (phasereco.h:110-122),
-    // and the flag map
-    for (int p = threadIdx.x; p < nbits; p += blockDim.x) {
-        const unsigned f = (flagbits[p >> 5] >> (p & 31)) & 1u;
+    if constexpr (MULTI)
+        cluster_sync_all(); // no CTA touches another's shared memory after this
+}
+
+// FP64 mean, consistency and phase of every point (phasereco.h:110-122) and
+// the flag map, once the walk is done.
+__global__ void __launch_bounds__(256) phase_final_kernel(const RecoJob* __restrict__ jobs)
+{
+    const RecoJob J = jobs[blockIdx.y];
+    const int W = J.W, H = J.H, e = J.De / 2;
+    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < W * H; p += gridDim.x * blockDim.x) {
+        int x = p % W, y = p / W; // FFT order -> the centred map
+        x -= x > -W / 2 + W - 1 ? W : 0;
+        y -= y > -H / 2 + H - 1 ? H : 0;
+        const float2 pf = J.pmap[(long long)(y + (H >> 1) + e) * (W + J.De) + x + (W >> 1) + e];
+        const bool f = !isnan(pf.x);
         J.flags[p] = f;
         if (!f)
             continue;
         const int n = J.cnt[p];
         if (n < 0) { // seed
-            J.phases[p] = make_double2(1.0, J.phf[p].y);
+            J.phases[p] = make_double2(1.0, pf.y);
             J.cons[p] = 1.0;
             continue;
         }
@@ -1116,56 +1160,57 @@ cudaError_t launch_offset_probe(const Geometry& g, const int* idx, long long n, 
 
 cudaError_t launch_phase_reco(const RecoJob* jobs_dev, int njobs, int max_W, int max_H, int max_De, cudaStream_t st)
 {
-    const int nv = (max_De + 1) * (max_De + 1);
-    reco_plan_kernel<<<dim3(1024, njobs), 256, 0, st>>>(jobs_dev);
+    const int nv = (max_De + 1) * (max_De + 1), nslots = (nv + 31) / 32 * 32;
+    spiral_plan_kernel<<<dim3(1216, njobs), 32 * kPlanWarps, sizeof(int) * nslots, st>>>(jobs_dev);
     note_launches(1);
-    reco_recent_kernel<<<dim3(1024, njobs), 256, 0, st>>>(jobs_dev);
-    note_launches(1);
-    reco_rlist_kernel<<<dim3(256, njobs), 256, 0, st>>>(jobs_dev);
-    note_launches(1);
-    const size_t smem = (sizeof(float2) + sizeof(int2)) * nv + sizeof(unsigned int) * (((size_t)max_W * max_H + 31) / 32);
-    // the limit is that of the largest frame and depth (the attribute is per
-    // function; a launch of another shape must never lower it under this one);
-    // the static shared memory (ring, phase cache) counts against it too
-    const size_t smem_max = (sizeof(float2) + sizeof(int2)) * 65 * 65
-                            + sizeof(unsigned int) * (((size_t)kMaxSide * kMaxSide + 31) / 32);
-    if (max_De < kClusterDepth) { // one CTA per job
-        cudaError_t e = cudaFuncSetAttribute(phase_pipe_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max);
+    const size_t smem = walk_smem(nslots);
+    // the limit is that of the largest depth (the attribute is per function; a
+    // launch of another shape must never lower it under this one)
+    const int smem_max = (int)walk_smem(kMaxWords * 32);
+    int ncta = walk_ctas(max_De);
+    cudaError_t e = cudaSuccess;
+    if (ncta > 1) {
+        // a cluster per job, or the largest that the GPU can place
+        e = cudaFuncSetAttribute(phase_walk_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
         if (e != cudaSuccess)
             return e;
-        phase_pipe_kernel<<<njobs, kRecoThreads, smem, st>>>(jobs_dev);
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.blockDim = dim3(kRecoThreads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        for (; ncta > 1; ncta /= 2) {
+            attr[0].val.clusterDim.x = ncta;
+            cfg.gridDim = dim3(ncta);
+            int nclusters = 0;
+            if (cudaOccupancyMaxActiveClusters(&nclusters, phase_walk_kernel<true>, &cfg) == cudaSuccess && nclusters >= 1)
+                break;
+            cudaGetLastError();
+        }
+        if (ncta > 1) {
+            cfg.gridDim = dim3(njobs * ncta);
+            e = cudaLaunchKernelEx(&cfg, phase_walk_kernel<true>, jobs_dev);
+            note_launches(1);
+        }
+    }
+    if (ncta <= 1) {
+        e = cudaFuncSetAttribute(phase_walk_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
+        if (e != cudaSuccess)
+            return e;
+        phase_walk_kernel<false><<<njobs, kRecoThreads, smem, st>>>(jobs_dev);
         note_launches(1);
-        return cudaGetLastError();
     }
-    cudaError_t e = cudaFuncSetAttribute(phase_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max);
-    if (e != cudaSuccess)
+    if (e != cudaSuccess || (e = cudaGetLastError()) != cudaSuccess)
         return e;
-    // one cluster per job: kWalkCtas CTAs, or the largest power of two below
-    // it that the GPU can place
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.blockDim = dim3(kRecoThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int ncta = kWalkCtas;
-    for (; ncta > 1; ncta /= 2) {
-        attr[0].val.clusterDim.x = ncta;
-        cfg.gridDim = dim3(ncta);
-        int nclusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&nclusters, phase_cluster_kernel, &cfg) == cudaSuccess && nclusters >= 1)
-            break;
-        cudaGetLastError();
-    }
-    attr[0].val.clusterDim.x = ncta;
-    cfg.gridDim = dim3(njobs * ncta);
-    e = cudaLaunchKernelEx(&cfg, phase_cluster_kernel, jobs_dev);
+    const int np = max_W * max_H;
+    phase_final_kernel<<<dim3((np + 255) / 256, njobs), 256, 0, st>>>(jobs_dev);
     note_launches(1);
-    return e != cudaSuccess ? e : cudaGetLastError();
+    return cudaGetLastError();
 }
 
 } // namespace smip_gpu

@@ -279,10 +279,10 @@ struct Reco {
     int* fring = nullptr;         // ring mode: per point the ring that set its phase (-1: none)
     int* rq = nullptr;            // ring mode: visit indices grouped by ring
     std::vector<int> roff;        // ring k: rq[roff[k] .. roff[k+1])
-    int4* pvis = nullptr;         // per point: first three visit indices, visit count
-    unsigned* rbits = nullptr;    // per visit: recent pair slots (bitmask)
-    int* rcount = nullptr;
-    unsigned short* rlist = nullptr;
+    uint4* rec = nullptr;         // per visit: its recent pairs
+    int4* meta = nullptr;         // per visit: where its point lies
+    int* oor = nullptr;
+    float2* pmap = nullptr;       // centred, padded phase map of the spiral walk
     int nvisits = 0;
     double2* phases = nullptr;
     float2* phf = nullptr;
@@ -297,10 +297,10 @@ struct Reco {
         dfree(visits);
         dfree(fring);
         dfree(rq);
-        dfree(pvis);
-        dfree(rbits);
-        dfree(rcount);
-        dfree(rlist);
+        dfree(rec);
+        dfree(meta);
+        dfree(oor);
+        dfree(pmap);
         dfree(phases);
         dfree(phf);
         dfree(sums);
@@ -310,6 +310,7 @@ struct Reco {
         dfree(flags);
         dfree(job);
     }
+    size_t map_bytes() const { return sizeof(float2) * (size_t)(g.W + g.De) * (g.H + g.De); }
     // Buffers and visit tables for radius `radius` (allocated once per stack,
     // the tables again only when the radius changes).
     int prepare(double radius, cudaStream_t st)
@@ -323,6 +324,8 @@ struct Reco {
             CUDA_TRY(cudaMalloc(&cons, sizeof(double) * np));
             CUDA_TRY(cudaMalloc(&flags, np));
             CUDA_TRY(cudaMalloc(&job, sizeof(RecoJob)));
+            CUDA_TRY(cudaMalloc(&oor, sizeof(int)));
+            CUDA_TRY(cudaMalloc(&pmap, map_bytes()));
         }
         if (radius != R) {
             std::vector<int> vring;
@@ -358,34 +361,14 @@ struct Reco {
             }
             dfree(visits);
             dfree(plan);
-            dfree(pvis);
-            dfree(rbits);
-            dfree(rcount);
-            dfree(rlist);
+            dfree(rec);
+            dfree(meta);
             CUDA_TRY(cudaMalloc(&visits, sizeof(int2) * v.size()));
             CUDA_TRY(cudaMemcpyAsync(visits, v.data(), sizeof(int2) * v.size(), cudaMemcpyHostToDevice, st));
             nvisits = (int)v.size();
-            const size_t nv = (size_t)(g.De + 1) * (g.De + 1);
-            CUDA_TRY(cudaMalloc(&plan, sizeof(float2) * nv * v.size()));
-            // each point's visits (the walk's order; a point may be visited again)
-            std::vector<int4> pv(np, make_int4(-1, -1, -1, 0));
-            const int pmin0 = -(g.W >> 1), pmin1 = -(g.H >> 1), pmax0 = g.W - 1 + pmin0, pmax1 = g.H - 1 + pmin1;
-            for (size_t q = 0; q < v.size(); ++q) {
-                const int2 w = v[q];
-                if (w.x < pmin0 || w.x > pmax0 || w.y < pmin1 || w.y > pmax1)
-                    continue;
-                int4& e = pv[(size_t)(w.x < 0 ? w.x + g.W : w.x) + (size_t)(w.y < 0 ? w.y + g.H : w.y) * g.W];
-                if (e.w == 0) e.x = (int)q;
-                else if (e.w == 1) e.y = (int)q;
-                else if (e.w == 2) e.z = (int)q;
-                ++e.w;
-            }
-            CUDA_TRY(cudaMalloc(&pvis, sizeof(int4) * np));
-            CUDA_TRY(cudaMemcpyAsync(pvis, pv.data(), sizeof(int4) * np, cudaMemcpyHostToDevice, st));
-            const size_t nwords = (nv + 31) / 32;
-            CUDA_TRY(cudaMalloc(&rbits, sizeof(unsigned) * nwords * v.size()));
-            CUDA_TRY(cudaMalloc(&rcount, sizeof(int) * v.size()));
-            CUDA_TRY(cudaMalloc(&rlist, sizeof(unsigned short) * kRecentMax * v.size()));
+            CUDA_TRY(cudaMalloc(&plan, sizeof(float2) * plan_row(g.De) * v.size()));
+            CUDA_TRY(cudaMalloc(&rec, sizeof(uint4) * kRecentMax * v.size()));
+            CUDA_TRY(cudaMalloc(&meta, sizeof(int4) * v.size()));
             R = radius;
         }
         if (mode == 1 && !fring)
@@ -398,8 +381,12 @@ struct Reco {
         if (int rc = prepare(radius, st))
             return rc;
         CUDA_TRY(cudaMemsetAsync(phases, 0, sizeof(double2) * np, st));
-        // the spiral walk's phase map marks a point without a phase by NaN (all bits set)
-        CUDA_TRY(cudaMemsetAsync(phf, mode == 1 ? 0 : 0xff, sizeof(float2) * np, st));
+        if (mode == 1) {
+            CUDA_TRY(cudaMemsetAsync(phf, 0, sizeof(float2) * np, st));
+        } else { // the spiral walk's phase map marks a point without a phase by NaN (all bits set)
+            CUDA_TRY(cudaMemsetAsync(pmap, 0xff, map_bytes(), st));
+            CUDA_TRY(cudaMemsetAsync(oor, 0, sizeof(int), st));
+        }
         CUDA_TRY(cudaMemsetAsync(cons, 0, sizeof(double) * np, st));
         RecoJob j;
         j.B = Bnorm;
@@ -416,10 +403,10 @@ struct Reco {
         j.cons = cons;
         j.flags = flags;
         j.err = err;
-        j.pvis = pvis;
-        j.rbits = rbits;
-        j.rcount = rcount;
-        j.rlist = rlist;
+        j.pmap = pmap;
+        j.rec = rec;
+        j.meta = meta;
+        j.oor = oor;
         CUDA_TRY(cudaMemcpyAsync(job, &j, sizeof(RecoJob), cudaMemcpyHostToDevice, st));
         if (mode == 1) {
             CUDA_TRY(launch_ring_reco(job, fring, rq, roff, g.W, g.H, st));

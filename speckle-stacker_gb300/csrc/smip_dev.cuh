@@ -504,6 +504,10 @@ __device__ __forceinline__ void dsmem_st_relaxed(uint32_t a, int v)
 {
     asm volatile("st.relaxed.cluster.shared::cluster.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
 }
+__device__ __forceinline__ void dsmem_st_f2(uint32_t a, float2 v)
+{
+    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(v.x), "f"(v.y) : "memory");
+}
 // Stores into another CTA's shared memory that complete a transaction count
 // on an mbarrier there (st.async): once the barrier's phase completes, a
 // thread of that CTA that waited on it sees the data.
@@ -517,6 +521,22 @@ __device__ __forceinline__ void dsmem_st_async_i(uint32_t a, int v, uint32_t bar
 {
     asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(a), "r"(v), "r"(bar)
                  : "memory");
+}
+// One arrival on a barrier of the cluster that also expects `bytes` of such
+// stores; relaxed: it orders nothing, the stores' completion does.
+__device__ __forceinline__ void dsmem_mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.relaxed.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+// Probe of a local barrier's phase that threads of the cluster complete.
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity)
+{
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok)
+                 : "r"(smem_u32(bar)), "r"(parity)
+                 : "memory");
+    return ok != 0;
 }
 // all threads of the cluster; every CTA's shared memory stays valid until
 // all have arrived

@@ -155,31 +155,30 @@ cudaError_t launch_bispec_normalize(const float2* B, const float2* C, double nfr
 cudaError_t launch_bispec_merge(float2* Bd, float2* Cd, const float2* Bs, const float2* Cs, long long n,
                                 cudaStream_t st);
 
-// Closure-phase recovery (one CTA per job).
+// Closure-phase recovery.
 struct RecoJob {
     const float2* B;     // normalised packed bispectrum
     const int2* visits;  // spiral visit list
     int nvisits;
     int W, H, De;
     double2* phases;     // W*H, FFT order
-    float2* phf;         // FP32 phases used along the chain (scratch)
-    float2* plan;        // [nvisits][(De+1)^2] unit phasors of B for every (visit, v)
+    float2* phf;         // FP32 phases used along the chain, FFT order (ring mode)
+    float2* pmap;        // FP32 phases used along the chain, centred with De / 2 points of padding, NaN: none (spiral walk)
+    float2* plan;        // [nvisits][plan_row(De)] unit phasors of B for every (visit, v); ring mode: [nvisits][(De+1)^2]
     float4* sums;        // per point: float-float phasor sums (re hi, re lo, im hi, im lo)
     int* cnt;            // per point: number of phasors (-1 for the seeds)
     double* cons;        // W*H
     unsigned char* flags;
     int* err;
-    // pipelined walk: per point its first three visit indices and its visit
-    // count (-1 padded); per visit the pairs whose u or v was visited within
-    // the last kRecoLag visits (bitmask over the (De+1)^2 pair slots), and
-    // their slots as a list (count -1: more than kRecentMax)
-    const int4* pvis;
-    unsigned* rbits;
-    int* rcount;
-    unsigned short* rlist;
+    // the spiral walk's visits (k_reco.cu, spiral_plan_kernel)
+    uint4* rec;          // [nvisits][kRecentMax] recent pairs
+    int4* meta;          // [nvisits]
+    int* oor;            // some pair's bispectrum element is out of range
 };
 constexpr int kRecoLag = 32;     // visits between a point's phase and the parallel stage's use of it
-constexpr int kRecentMax = 64;   // recent pairs per visit the serial warp takes from a list
+constexpr int kRecentMax = 64;   // recent pairs per visit: at most 32 by u and 32 by v
+// pair slots of a plan row: (De+1)^2 rounded up to whole warps (16-byte aligned rows)
+constexpr size_t plan_row(int De) { return ((size_t)(De + 1) * (De + 1) + 31) / 32 * 32; }
 cudaError_t launch_phase_reco(const RecoJob* jobs_dev, int njobs, int max_W, int max_H, int max_De, cudaStream_t st);
 // Ring-parallel estimator (opt-in, not the reference's): rq holds the spiral's
 // visit indices grouped by ring, ring k at [roff[k], roff[k+1]); fring: W*H ints.
