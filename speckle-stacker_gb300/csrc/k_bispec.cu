@@ -58,14 +58,44 @@ cudaError_t launch_bounded_wait_probe(int* err, const int* never, double timeout
 }
 
 // ------------------------------------------------------- normalise, merge
-// (B - C) / n: the difference is exact in FP64; a multiply by 1/n instead of
-// a divide keeps the FP64 pipe's share small (GB300's FP64 rate is low).
-__global__ void bispec_normalize_kernel(const float2* __restrict__ B, const float2* __restrict__ C, double inv_n,
-                                        long long count, float2* __restrict__ out)
+// (B - C) / n, rounded once: the difference is formed exactly as a float pair
+// and multiplied by 1/n as one, on the FP32 pipes (GB300's FP64 rate bound this
+// kernel: 351 us at 256 x 256, d = 32, 1.3 TB/s; now HBM does).  Values near the
+// ends of the FP32 range, infinities and NaN take the FP64 form.
+// (a call, so that the compiler does not compute it beside the other form)
+__device__ __noinline__ float normalized_f64(float b, float c, double inv_n)
 {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < count; i += (long long)gridDim.x * blockDim.x) {
-        const float2 b = B[i], c = C[i];
-        out[i] = make_float2((float)(((double)b.x - (double)c.x) * inv_n), (float)(((double)b.y - (double)c.y) * inv_n));
+    return (float)(((double)b - (double)c) * inv_n);
+}
+__device__ __forceinline__ float normalized(float b, float c, float ih, float il, double inv_n)
+{
+    float s, e;
+    two_sum(b, -c, s, e);
+    const float p = __fmul_rn(s, ih);
+    const float r = __fadd_rn(p, fmaf(e, ih, fmaf(s, il, fmaf(s, ih, -p))));
+    const float m = fabsf(s);
+    if (m <= 1e37f && (m >= 1e-24f || m == 0.f))
+        return r;
+    return normalized_f64(b, c, inv_n);
+}
+
+__global__ void __launch_bounds__(256) bispec_normalize_kernel(const float2* __restrict__ B, const float2* __restrict__ C,
+                                                               double inv_n, long long count, float2* __restrict__ out)
+{
+    const float ih = (float)inv_n, il = (float)(inv_n - (double)ih);
+    const long long step = (long long)gridDim.x * blockDim.x, pairs = count / 2; // the arrays are 256-byte aligned
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < pairs; i += step) {
+        const float4 b = __ldcs(reinterpret_cast<const float4*>(B) + i), c = __ldcs(reinterpret_cast<const float4*>(C) + i);
+        float4 o;
+        o.x = normalized(b.x, c.x, ih, il, inv_n);
+        o.y = normalized(b.y, c.y, ih, il, inv_n);
+        o.z = normalized(b.z, c.z, ih, il, inv_n);
+        o.w = normalized(b.w, c.w, ih, il, inv_n);
+        reinterpret_cast<float4*>(out)[i] = o;
+    }
+    if ((count & 1) && blockIdx.x == 0 && threadIdx.x == 0) {
+        const float2 b = B[count - 1], c = C[count - 1];
+        out[count - 1] = make_float2(normalized(b.x, c.x, ih, il, inv_n), normalized(b.y, c.y, ih, il, inv_n));
     }
 }
 
@@ -89,7 +119,10 @@ __global__ void bispec_merge_kernel(float2* __restrict__ Bd, float2* __restrict_
 cudaError_t launch_bispec_normalize(const float2* B, const float2* C, double nframes, long long n, float2* out,
                                     cudaStream_t st)
 {
-    bispec_normalize_kernel<<<2048, 256, 0, st>>>(B, C, 1.0 / nframes, n, out); note_launches(1);
+    // eight blocks an SM, a few pairs a thread; fewer blocks for a small array
+    const long long blocks = (n / 2 + 255) / 256;
+    bispec_normalize_kernel<<<(int)(blocks < 1 ? 1 : blocks > 152 * 8 * 4 ? 152 * 8 * 4 : blocks), 256, 0, st>>>(B, C, 1.0 / nframes, n, out);
+    note_launches(1);
     return cudaGetLastError();
 }
 
