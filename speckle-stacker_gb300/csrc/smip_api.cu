@@ -199,12 +199,19 @@ int make_gen_tw(int L, GenTw* t)
         tdf[k].h = t32[k];
         tdf[k].l = make_float2((float)(t64[k].x - (double)hx), (float)(t64[k].y - (double)hy));
     }
-    // the passes' index map (GenPlan::map): j | e0 << 16 per pass and output
+    // the passes' index map (GenPlan::map)
     const GenPlan p = make_gen_plan(L);
     std::vector<unsigned> map((size_t)p.nf * L);
     for (int f = 0, Ns = 1; f < p.nf; Ns *= p.fac[f], ++f) {
         const int R = p.fac[f], step = L / (Ns * R);
-        for (int o = 0; o < L; ++o) {
+        if (gen_butterfly(R)) { // per butterfly: its first output and twiddle exponent
+            for (int j = 0; j < L / R; ++j) {
+                const int k = j % Ns;
+                map[(size_t)f * L + j] = (unsigned)((j - k) * R + k) | ((unsigned)(k * step) << 16);
+            }
+            continue;
+        }
+        for (int o = 0; o < L; ++o) { // per output: its first input and exponent step
             const int k = o % Ns, t = o / Ns, q = t % R;
             map[(size_t)f * L + o] = (unsigned)((t / R) * Ns + k) | ((unsigned)((k + q * Ns) * step) << 16);
         }

@@ -26,10 +26,13 @@ struct GenPlan {
     int L;
     int nf;
     int fac[kMaxFactors];
-    // per pass f and output o: j | e0 << 16, the pass's input index and twiddle
-    // exponent step (k_fftg.cu), nf x L entries in device memory (null: computed)
+    // per pass f, nf x L entries in device memory (null: computed): a butterfly
+    // j's first output | twiddle exponent << 16, or for a larger prime an output
+    // o's input index j | twiddle exponent step << 16 (k_fftg.cu)
     const unsigned* map = nullptr;
 };
+// radices that a thread transforms in registers
+constexpr bool gen_butterfly(int R) { return R <= 5 || R == 7 || R == 8; }
 GenPlan make_gen_plan(int L);
 constexpr int kRowBlock = 16;     // rows per CTA in the row passes
 constexpr int kColLines = 8;      // frames per FFT pass in the column kernel
