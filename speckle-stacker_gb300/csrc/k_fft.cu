@@ -53,9 +53,10 @@ __device__ __forceinline__ float2 df_round(const dfc& v) { return make_float2(v.
 template <typename T>
 __global__ void __launch_bounds__(256, 4) row_pass_kernel(const T* __restrict__ frames, long long fstride, int logW, int H,
                                                         int hw, dfc* __restrict__ Gt, const dfc* __restrict__ tw_g,
-                                                        T* __restrict__ copy_out)
+                                                        T* __restrict__ copy_out, float* __restrict__ rowsq)
 {
     extern __shared__ dfc smdf[];
+    float sq = 0.f; // of this thread's pixels, for the correlation's error bound (k_xcorr.cu)
     const int W = 1 << logW;
     dfc* tw = smdf;                                // W - 1, stage-packed (+1 spare)
     dfc* lines = smdf + W;                         // [kRowBlock/2][pad8(W) + 1]
@@ -100,16 +101,20 @@ __global__ void __launch_bounds__(256, 4) row_pass_kernel(const T* __restrict__ 
                 dfc d;
                 d.h = make_float2((float)p0[e], (float)p1[e]);
                 d.l = make_float2(0.f, 0.f);
+                sq = fmaf(d.h.x, d.h.x, fmaf(d.h.y, d.h.y, sq));
                 L[pad8(bitrev(x0 + e, logW))] = d;
             }
         }
     } else {
         for (int idx = threadIdx.x; idx < kRowBlock * W; idx += blockDim.x) {
-            put(idx, pix_df(fr, idx));
+            const float2 v = pix_df(fr, idx);
+            sq = fmaf(v.x, v.x, sq);
+            put(idx, v);
             if (co)
                 co[idx] = fr[idx];
         }
     }
+    store_block_sum(sq, rowsq + (long long)f * gridDim.x + blockIdx.x);
     __syncthreads();
     fft_passes(lines, logW, kRowBlock / 2, LW, tw, kTwLog, -1);
     dfc* out = Gt + (long long)f * hw * H;
@@ -134,11 +139,15 @@ __global__ void __launch_bounds__(256, 4) row_pass_kernel(const T* __restrict__ 
 // One CTA per (a, chunk of frames).  Float-float forward FFT along y gives
 // Fm(a, y) = F(-a, y); writes S (rounded to FP32), accumulates |F|^2 in float-float
 // (frame order), and for the correlation computes the FP32 inverse
-// y-transform of conj(R) * Fm into T.
-__global__ void __launch_bounds__(256) col_pass_kernel(int mode, const dfc* __restrict__ Gt, float2* __restrict__ S,
-                                                        const float2* __restrict__ Rbuf, float2* __restrict__ Rout,
+// y-transform of conj(R) * Fm into T.  first: frame 0 of the batch is the
+// reference; every CTA transforms its column of it (a line more to a chunk of
+// 16, instead of a launch of one line per CTA that the others would wait for),
+// and the first chunk's write it to R for the later batches.  first = 2: frame 0
+// is the reference and its spectrum is in R already.
+__global__ void __launch_bounds__(256) col_pass_kernel(const dfc* __restrict__ Gt, float2* __restrict__ S,
+                                                        float2* __restrict__ Rbuf,
                                                         float2* __restrict__ T, double* __restrict__ Ppart,
-                                                        int nframes, int fpc, int skip_xcorr_frame0, int logH, int hw,
+                                                        int nframes, int fpc, int first, int logH, int hw,
                                                         const dfc* __restrict__ twdf_g, const float2* __restrict__ tw_g)
 {
     extern __shared__ dfc smdf[];
@@ -157,11 +166,22 @@ __global__ void __launch_bounds__(256) col_pass_kernel(int mode, const dfc* __re
     const long long gstride = (long long)hw * H;
     load_twiddles_packed(twd, twdf_g, logH, kTwLog);
     load_twiddles_packed(tw, tw_g, logH, kTwLog);
-    if (mode == 0)
-        for (int y = threadIdx.x; y < H; y += blockDim.x) {
+    for (int y = threadIdx.x; y < H; y += blockDim.x) {
+        if (first != 1)
             R[y] = Rbuf[(long long)a * H + y];
-            pacc[y] = make_float2(0.f, 0.f);
+        pacc[y] = make_float2(0.f, 0.f);
+    }
+    if (first == 1) {
+        for (int y = threadIdx.x; y < H; y += blockDim.x)
+            L1[pad8(bitrev(y, logH))] = Gt[(long long)a * H + y];
+        __syncthreads();
+        fft_passes(L1, logH, 1, LH, twd, kTwLog, -1);
+        for (int y = threadIdx.x; y < H; y += blockDim.x) {
+            R[y] = df_round(L1[pad8(y)]);
+            if (chunk == 0)
+                Rbuf[(long long)a * H + y] = R[y];
         }
+    }
     for (int f0 = fbeg; f0 < fend; f0 += kColLines) {
         const int nl = min(kColLines, fend - f0);
         __syncthreads();
@@ -177,11 +197,6 @@ __global__ void __launch_bounds__(256) col_pass_kernel(int mode, const dfc* __re
         }
         __syncthreads();
         fft_passes(L1, logH, nl, LH, twd, kTwLog, -1);
-        if (mode == 1) { // reference spectrum only
-            for (int y = threadIdx.x; y < H; y += blockDim.x)
-                Rout[(long long)a * H + y] = df_round(L1[pad8(y)]);
-            return;
-        }
         for (int idx = threadIdx.x; idx < nl * H; idx += blockDim.x) {
             const int l = idx >> logH, c = idx & (H - 1);
             S[(f0 + l) * gstride + (long long)a * H + c] = df_round(L1[l * LH + pad8((c + H / 2) & (H - 1))]);
@@ -213,7 +228,7 @@ __global__ void __launch_bounds__(256) col_pass_kernel(int mode, const dfc* __re
         fft_passes(L2, logH, nl, LH, tw, kTwLog, +1);
         for (int idx = threadIdx.x; idx < nl * H; idx += blockDim.x) {
             const int l = idx >> logH, y = idx & (H - 1);
-            if (skip_xcorr_frame0 && f0 + l == 0)
+            if (first && f0 + l == 0)
                 continue;
             T[(f0 + l) * gstride + (long long)a * H + y] = L2[l * LH + pad8(y)];
         }
@@ -345,8 +360,10 @@ static size_t col_pass_smem(int H)
 }
 static size_t xcorr_rows_smem(int W) { return sizeof(float2) * (W + (W / 2 + 1) * (kRowBlock + 1) + (kRowBlock / 2) * pad8(W)); }
 
+int row_blocks(const Geometry& g) { return g.generic ? gen_row_blocks(g) : g.H / kRowBlock; }
+
 cudaError_t launch_row_pass(int dtype, const void* frames, long long fstride, int nframes, const Geometry& g, dfc* Gt,
-                            const dfc* twdf, cudaStream_t st, void* copy_out)
+                            float* rowsq, const dfc* twdf, cudaStream_t st, void* copy_out)
 {
     const dim3 grid(g.H / kRowBlock, nframes);
     const size_t smem = row_pass_smem(g.W), smem_max = row_pass_smem(1 << kMaxLog);
@@ -355,40 +372,37 @@ cudaError_t launch_row_pass(int dtype, const void* frames, long long fstride, in
     case 0:
         if ((e = allow_smem(row_pass_kernel<uint8_t>, smem_max)) != cudaSuccess) return e;
         row_pass_kernel<uint8_t><<<grid, 256, smem, st>>>((const uint8_t*)frames, fstride, g.logW, g.H, g.hw, Gt, twdf,
-                                                          (uint8_t*)copy_out);
+                                                          (uint8_t*)copy_out, rowsq);
         break;
     case 1:
         if ((e = allow_smem(row_pass_kernel<uint16_t>, smem_max)) != cudaSuccess) return e;
         row_pass_kernel<uint16_t><<<grid, 256, smem, st>>>((const uint16_t*)frames, fstride, g.logW, g.H, g.hw, Gt, twdf,
-                                                           (uint16_t*)copy_out);
+                                                           (uint16_t*)copy_out, rowsq);
         break;
     case 2:
         if ((e = allow_smem(row_pass_kernel<float>, smem_max)) != cudaSuccess) return e;
         row_pass_kernel<float><<<grid, 256, smem, st>>>((const float*)frames, fstride, g.logW, g.H, g.hw, Gt, twdf,
-                                                        (float*)copy_out);
+                                                        (float*)copy_out, rowsq);
         break;
     default:
         if ((e = allow_smem(row_pass_kernel<double>, smem_max)) != cudaSuccess) return e;
         row_pass_kernel<double><<<grid, 256, smem, st>>>((const double*)frames, fstride, g.logW, g.H, g.hw, Gt, twdf,
-                                                         (double*)copy_out);
+                                                         (double*)copy_out, rowsq);
         break;
     }
     note_launches(1);
     return cudaGetLastError();
 }
 
-cudaError_t launch_col_pass(int mode, const dfc* Gt, float2* S, const float2* Rbuf, float2* Rout, float2* T,
-                            double* Ppart, int nframes, int fpc, int skip_xcorr_frame0, const Geometry& g,
-                            const dfc* twdf, const float2* tw, cudaStream_t st)
+cudaError_t launch_col_pass(const dfc* Gt, float2* S, float2* Rbuf, float2* T, double* Ppart, int nframes, int fpc,
+                            int first, const Geometry& g, const dfc* twdf, const float2* tw, cudaStream_t st)
 {
-    const int nchunks = mode == 1 ? 1 : (nframes + fpc - 1) / fpc;
-    const dim3 grid(g.hw, nchunks);
+    const dim3 grid(g.hw, (nframes + fpc - 1) / fpc);
     const size_t smem = col_pass_smem(g.H);
     cudaError_t e = allow_smem(col_pass_kernel, col_pass_smem(1 << kMaxLog));
     if (e != cudaSuccess)
         return e;
-    col_pass_kernel<<<grid, 256, smem, st>>>(mode, Gt, S, Rbuf, Rout, T, Ppart, mode == 1 ? 1 : nframes, fpc,
-                                             skip_xcorr_frame0, g.logH, g.hw, twdf, tw);
+    col_pass_kernel<<<grid, 256, smem, st>>>(Gt, S, Rbuf, T, Ppart, nframes, fpc, first, g.logH, g.hw, twdf, tw);
     note_launches(1);
     return cudaGetLastError();
 }

@@ -284,9 +284,11 @@ __device__ __forceinline__ float2 dfc_round(const dfc& v) { return make_float2(v
 template <typename T>
 __global__ void __launch_bounds__(256, 4) gen_row_kernel(const T* __restrict__ frames, long long fstride, int H, int hw,
                                                       int rb, const GenPlan pw, const dfc* __restrict__ tw_g,
-                                                      dfc* __restrict__ Gt, T* __restrict__ copy_out)
+                                                      dfc* __restrict__ Gt, T* __restrict__ copy_out,
+                                                      float* __restrict__ rowsq)
 {
     extern __shared__ dfc smg[];
+    float sq = 0.f; // of this thread's pixels, for the correlation's error bound (k_xcorr.cu)
     const int W = pw.L;
     dfc* tw = smg;
     dfc* X = tw + W;
@@ -304,6 +306,7 @@ __global__ void __launch_bounds__(256, 4) gen_row_kernel(const T* __restrict__ f
         dfc d;
         d.h = make_float2(p0.x, p1.x);
         d.l = make_float2(p0.y, p1.y);
+        sq = fmaf(p0.x, p0.x, fmaf(p1.x, p1.x, sq));
         X[i] = d;
         if (co) {
             co[at] = fr[at];
@@ -311,6 +314,7 @@ __global__ void __launch_bounds__(256, 4) gen_row_kernel(const T* __restrict__ f
                 co[at + W] = fr[at + W];
         }
     }
+    store_block_sum(sq, rowsq + (long long)f * gridDim.x + blockIdx.x);
     __syncthreads();
     const dfc* Z = stockham(X, Y, pw, nl, W, tw, -1);
     dfc* out = Gt + (long long)f * hw * H;
@@ -336,11 +340,12 @@ __global__ void __launch_bounds__(256, 4) gen_row_kernel(const T* __restrict__ f
 // transform along y gives F(-a, y); writes S[f][a][c] = F(-a, c - H/2) (row
 // pitch Hs, rounded to FP32), the power partials |F|^2 summed in float-float
 // in frame order, and the FP32 inverse y-transform of conj(R) * F into T.
-// mode 1: frame 0 only, its spectrum F(-a, y) into Rout (y in natural order).
-__global__ void __launch_bounds__(256, 4) gen_col_kernel(int mode, const dfc* __restrict__ Gt, float2* __restrict__ S,
-                                                      int Hs, const float2* __restrict__ Rbuf, float2* __restrict__ Rout,
+// first: frame 0 is the reference, whose column every CTA transforms first
+// (k_fft.cu).
+__global__ void __launch_bounds__(256, 4) gen_col_kernel(const dfc* __restrict__ Gt, float2* __restrict__ S,
+                                                      int Hs, float2* __restrict__ Rbuf,
                                                       float2* __restrict__ T, double* __restrict__ Ppart, int nframes,
-                                                      int fpc, int skip_xcorr_frame0, int hw, int cl, const GenPlan ph,
+                                                      int fpc, int first, int hw, int cl, const GenPlan ph,
                                                       const dfc* __restrict__ twd_g, const float2* __restrict__ tw_g)
 {
     extern __shared__ dfc smg[];
@@ -360,11 +365,22 @@ __global__ void __launch_bounds__(256, 4) gen_col_kernel(int mode, const dfc* __
     const int hh = H / 2;
     load_table(twd, twd_g, H);
     load_table(tw, tw_g, H);
-    if (mode == 0)
-        for (int y = threadIdx.x; y < H; y += blockDim.x) {
+    for (int y = threadIdx.x; y < H; y += blockDim.x) {
+        if (first != 1)
             R[y] = Rbuf[(long long)a * H + y];
-            pacc[y] = make_float2(0.f, 0.f);
+        pacc[y] = make_float2(0.f, 0.f);
+    }
+    if (first == 1) {
+        for (int y = threadIdx.x; y < H; y += blockDim.x)
+            X[y] = Gt[(long long)a * H + y];
+        __syncthreads();
+        const dfc* Fr = stockham(X, Y, ph, 1, H, twd, -1);
+        for (int y = threadIdx.x; y < H; y += blockDim.x) {
+            R[y] = dfc_round(Fr[y]);
+            if (chunk == 0)
+                Rbuf[(long long)a * H + y] = R[y];
         }
+    }
     for (int f0 = fbeg; f0 < fend; f0 += cl) {
         const int nl = min(cl, fend - f0);
         __syncthreads();
@@ -377,11 +393,6 @@ __global__ void __launch_bounds__(256, 4) gen_col_kernel(int mode, const dfc* __
         // the FP32 transform's buffers: the other one, then Fm's own
         float2* X2 = reinterpret_cast<float2*>(Fm == X ? Y : X);
         float2* Y2 = reinterpret_cast<float2*>(Fm);
-        if (mode == 1) {
-            for (int y = threadIdx.x; y < H; y += blockDim.x)
-                Rout[(long long)a * H + y] = dfc_round(Fm[y]);
-            return;
-        }
         for (int i = threadIdx.x; i < nl * H; i += blockDim.x) {
             const int l = i / H, c = i - l * H;
             int y = c - hh;
@@ -415,7 +426,7 @@ __global__ void __launch_bounds__(256, 4) gen_col_kernel(int mode, const dfc* __
         const float2* Tz = stockham(X2, Y2, ph, nl, H, tw, +1);
         for (int i = threadIdx.x; i < nl * H; i += blockDim.x) {
             const int l = i / H, y = i - l * H;
-            if (skip_xcorr_frame0 && f0 + l == 0)
+            if (first && f0 + l == 0)
                 continue;
             T[(f0 + l) * gstride + (long long)a * H + y] = Tz[i];
         }
@@ -546,9 +557,10 @@ template <typename K> static cudaError_t allow(K kern, size_t bytes)
 }
 
 size_t gen_max_smem() { return kGenSmem; }
+int gen_row_blocks(const Geometry& g) { return (g.H + row_block(g.W) - 1) / row_block(g.W); }
 
 cudaError_t launch_gen_row_pass(int dtype, const void* frames, long long fstride, int nframes, const Geometry& g,
-                                dfc* Gt, const dfc* twW, cudaStream_t st, void* copy_out)
+                                dfc* Gt, float* rowsq, const dfc* twW, cudaStream_t st, void* copy_out)
 {
     const int rb = row_block(g.W);
     const dim3 grid((g.H + rb - 1) / rb, nframes);
@@ -558,7 +570,7 @@ cudaError_t launch_gen_row_pass(int dtype, const void* frames, long long fstride
     if ((e = allow(gen_row_kernel<TY>, kGenSmem)) != cudaSuccess)                                                 \
         return e;                                                                                                  \
     gen_row_kernel<TY><<<grid, 256, smem, st>>>((const TY*)frames, fstride, g.H, g.hw, rb, g.pW, twW, Gt,         \
-                                                (TY*)copy_out);
+                                                (TY*)copy_out, rowsq);
     switch (dtype) {
     case 0: SMIP_GEN_ROW(uint8_t) break;
     case 1: SMIP_GEN_ROW(uint16_t) break;
@@ -570,18 +582,15 @@ cudaError_t launch_gen_row_pass(int dtype, const void* frames, long long fstride
     return cudaGetLastError();
 }
 
-cudaError_t launch_gen_col_pass(int mode, const dfc* Gt, float2* S, const float2* Rbuf, float2* Rout, float2* T,
-                                double* Ppart, int nframes, int fpc, int skip_xcorr_frame0, const Geometry& g,
-                                const dfc* twH, const float2* twH32, cudaStream_t st)
+cudaError_t launch_gen_col_pass(const dfc* Gt, float2* S, float2* Rbuf, float2* T, double* Ppart, int nframes, int fpc,
+                                int first, const Geometry& g, const dfc* twH, const float2* twH32, cudaStream_t st)
 {
-    const int nchunks = mode == 1 ? 1 : (nframes + fpc - 1) / fpc;
     const int cl = col_lines(g.H);
-    const dim3 grid(g.hw, nchunks);
+    const dim3 grid(g.hw, (nframes + fpc - 1) / fpc);
     cudaError_t e = allow(gen_col_kernel, kGenSmem);
     if (e != cudaSuccess)
         return e;
-    gen_col_kernel<<<grid, 256, col_smem(g.H, cl), st>>>(mode, Gt, S, g.Hs, Rbuf, Rout, T, Ppart,
-                                                         mode == 1 ? 1 : nframes, fpc, skip_xcorr_frame0, g.hw, cl,
+    gen_col_kernel<<<grid, 256, col_smem(g.H, cl), st>>>(Gt, S, g.Hs, Rbuf, T, Ppart, nframes, fpc, first, g.hw, cl,
                                                          g.pH, twH, twH32);
     note_launches(1);
     return cudaGetLastError();

@@ -133,84 +133,100 @@ __device__ void exact_corr_multi(const T* __restrict__ ref, const T* __restrict_
         for (int c = 0; c < kMulti; ++c)
             red[c * 32 + w] = acc[c];
     __syncthreads();
-#pragma unroll
-    for (int c = 0; c < kMulti; ++c) {
+    if (threadIdx.x < kMulti) { // one thread each: GB300's FP64 rate is low
         A t = 0;
         for (int i = 0; i < nw; ++i)
-            t += red[c * 32 + i];
-        out[c] = t;
+            t += red[threadIdx.x * 32 + i];
+        red[threadIdx.x * 32] = t;
     }
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < kMulti; ++c)
+        out[c] = red[c * 32];
     __syncthreads();
 }
 
+// Sum of squares over one frame in FP64, by all threads.
+template <typename T> __device__ double frame_sumsq(const T* __restrict__ p, int n, double* red)
+{
+    double s = 0.0;
+    for (int i = threadIdx.x; i < n; i += blockDim.x)
+        s += (double)p[i] * (double)p[i];
+    return block_sum(s, red);
+}
+
+// A frame's sum of squares from the row pass's sums of its row blocks: FP32,
+// within 1e-3 of the exact one, which the bound below allows for.  Every warp
+// forms it for itself (the same additions, so the same bits).
+__device__ float frame_norm(const float* __restrict__ part, int nsq)
+{
+    float s = 0.f;
+    for (int i = threadIdx.x & 31; i < nsq; i += 32)
+        s += part[i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+        s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+}
+// sums at the ends of the FP32 range are formed again in FP64
+__device__ __forceinline__ bool norm_ok(float s) { return s > 1e-25f && s < 1e30f; }
+
+// Bound by latency: a frame's pixels are read only where more than one position
+// lies within the bound of the peak (few frames), and the norms come from the row
+// pass.  With the frame read for its norm and the peak always re-scored, 2000
+// frames of 256 x 256 took 369 us instead of 102.
+// One CTA per frame.  rowsq: nsq sums per frame; refsq: those of the reference,
+// or null (its sum of squares is *ref_sq then).  The stack's frame 0 (first) is
+// the reference itself: it shifts by (0, 0), and its CTA writes *ref_sq for the
+// later batches.
 template <typename T>
 __global__ void __launch_bounds__(kShiftThreads) xcorr_shift_kernel(const float* __restrict__ corr,
                                                                      const float* __restrict__ rowmax,
                                                                      const T* __restrict__ frames, long long fstride,
-                                                                     const T* __restrict__ ref, const double* ref_sq,
-                                                                     int first_is_frame0, int W, int logW, int H,
+                                                                     const T* __restrict__ ref,
+                                                                     const float* __restrict__ rowsq, int nsq,
+                                                                     const float* __restrict__ refsq, double* ref_sq,
+                                                                     int first, int W, int logW, int H,
                                                                      double err_stages, int* __restrict__ shifts)
 {
     using A = typename ExactAcc<T>::type;
     __shared__ A redM[kMulti * 32];
-    __shared__ A redA1[32];
-    __shared__ float redF[32];
+    __shared__ double redD[32];
     __shared__ int cand[kMaxCand];
     __shared__ int ncand;
     const int f = blockIdx.x;
-    if (first_is_frame0 && f == 0) {
+    const int n = W * H;
+    if (first && f == 0) {
+        const float s32 = frame_norm(refsq, nsq);
+        const double s = norm_ok(s32) ? (double)s32 : frame_sumsq(ref, n, redD);
         if (threadIdx.x == 0) {
+            *ref_sq = s;
             shifts[0] = 0;
             shifts[1] = 0;
         }
         return;
     }
-    const int n = W * H;
     const float* c = corr + (long long)f * n;
     const float* rm = rowmax + (long long)f * H;
     const T* fr = frames + (long long)f * fstride;
-    // ||frame||^2 (the frame uses vector loads when its address allows) and
-    // the FP32 peak from the rows' maxima
-    A sqa = 0; // exact (u64) for integer frames, FP64 for float frames
+    // the norms and the FP32 peak from the rows' maxima, by every warp
     float mx = -INFINITY;
-    for (int y = threadIdx.x; y < H; y += blockDim.x)
+    for (int y = threadIdx.x & 31; y < H; y += 32)
         mx = fmaxf(mx, rm[y]);
-    constexpr int PV = sizeof(T) == 8 ? 2 : 4;           // pixels per frame vector load
-    const bool vec = (reinterpret_cast<uintptr_t>(fr) & 15) == 0;
-    for (int p = threadIdx.x * 4; p < n; p += blockDim.x * 4) {
-        if (vec) {
-#pragma unroll
-            for (int q = 0; q < 4; q += PV) {
-                T px[PV];
-                if (sizeof(T) == 1)
-                    *reinterpret_cast<uint32_t*>(px) = *reinterpret_cast<const uint32_t*>(fr + p + q);
-                else if (sizeof(T) == 2)
-                    *reinterpret_cast<uint2*>(px) = *reinterpret_cast<const uint2*>(fr + p + q);
-                else
-                    *reinterpret_cast<uint4*>(px) = *reinterpret_cast<const uint4*>(fr + p + q);
-#pragma unroll
-                for (int e = 0; e < PV; ++e)
-                    sqa += mul_exact<A>(px[e], px[e]);
-            }
-        } else {
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-                sqa += mul_exact<A>(fr[p + e], fr[p + e]);
-        }
-    }
-    const double sq = (double)block_sum(sqa, redA1);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0)
-        redF[threadIdx.x >> 5] = mx;
-    __syncthreads();
-    mx = redF[0];
-    for (int i = 1; i < (int)(blockDim.x >> 5); ++i)
-        mx = fmaxf(mx, redF[i]);
-    const double tau = 8.0 * 5.9604644775390625e-08 * err_stages * sqrt(*ref_sq * sq) * (double)n;
-    const float thr = (float)((double)mx - tau);
+    const float sq = frame_norm(rowsq + (long long)f * nsq, nsq);
+    const float rsq = refsq ? frame_norm(refsq, nsq) : (float)*ref_sq;
+    float thr;
+    if (norm_ok(sq) && norm_ok(rsq)) { // FP32, rounded down
+        thr = __fsub_rd(mx, 1.003f * 8.0f * 5.9604644775390625e-08f * (float)err_stages * sqrtf(rsq) * sqrtf(sq) * (float)n);
+    } else {
+        const double sqd = norm_ok(sq) ? (double)sq : frame_sumsq(fr, n, redD);
+        const double rsqd = norm_ok(rsq) ? (double)rsq : refsq ? frame_sumsq(ref, n, redD) : *ref_sq;
+        const double tau = 1.002 * 8.0 * 5.9604644775390625e-08 * err_stages * sqrt(rsqd * sqd) * (double)n;
+        thr = (float)((double)mx - tau);
+    }
 
     A best = 0;
     int best_idx = -1;
@@ -265,7 +281,9 @@ __global__ void __launch_bounds__(kShiftThreads) xcorr_shift_kernel(const float*
     __syncthreads();
     const int total_cand = ncand;
     __syncthreads();
-    if (total_cand <= kMaxCand) {
+    if (total_cand == 1) { // nothing within the bound of the peak but the peak
+        best_idx = cand[0];
+    } else if (total_cand <= kMaxCand) {
         rescore(total_cand);
     } else {
         // More candidates than the list holds: windows of blockDim.x
@@ -313,7 +331,10 @@ __device__ __forceinline__ double abs_px(double v) { return fabs(v); }
 // Integer frames (u64 sums) are exact in any order, so the batch's frames are
 // also split over gridDim.y CTAs whose partial sums are added atomically;
 // float frames (f64 sums) keep one CTA per pixel block, frames in order.
-template <typename T, typename A>
+// kU frames' loads are in flight at a time; float frames, whose one chain of
+// FP64 additions per pixel is the time, take more of them, smaller blocks and no
+// branch per frame (150 frames of 99 x 75: 37.2 -> 19.6 us).
+template <typename T, typename A, int kU>
 __global__ void __launch_bounds__(256) saa_add_kernel(A* __restrict__ sum, const T* __restrict__ frames,
                                                       long long fstride, int nframes, int first_is_frame0,
                                                       const int* __restrict__ shifts, int W, int H)
@@ -330,19 +351,18 @@ __global__ void __launch_bounds__(256) saa_add_kernel(A* __restrict__ sum, const
         const int y = p / W, x = p - y * W;
         A acc = kExact ? A(0) : sum[p];
         int f = fb;
-        for (; f + 8 <= fe; f += 8) { // eight independent loads in flight, added in frame order
-            A v[8];
-            bool in[8];
+        for (; f + kU <= fe; f += kU) { // independent loads in flight, added in frame order
+            T v[kU];
+            bool in[kU];
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
+            for (int q = 0; q < kU; ++q) {
                 const int xs = x + sh[f - fb + q].x, ys = y + sh[f - fb + q].y;
                 in[q] = xs >= 0 && xs < W && ys >= 0 && ys < H;
-                v[q] = in[q] ? (A)frames[(long long)(f + q) * fstride + ys * W + xs] : (A)0;
+                v[q] = in[q] ? frames[(long long)(f + q) * fstride + ys * W + xs] : T(0);
             }
 #pragma unroll
-            for (int q = 0; q < 8; ++q)
-                if (in[q])
-                    acc += (first_is_frame0 && f + q == 0) ? v[q] : abs_px(v[q]);
+            for (int q = 0; q < kU; ++q) // outside the frame: zero, which changes no sum
+                acc += (first_is_frame0 && f + q == 0) ? (A)v[q] : abs_px((A)v[q]);
         }
         for (; f < fe; ++f) {
             const int xs = x + sh[f - fb].x, ys = y + sh[f - fb].y;
@@ -358,23 +378,9 @@ __global__ void __launch_bounds__(256) saa_add_kernel(A* __restrict__ sum, const
     }
 }
 
-template <typename T>
-__global__ void sumsq_kernel(const T* __restrict__ fr, long long n, double* out)
-{
-    __shared__ double red[32];
-    double s = 0.0;
-    for (long long p = threadIdx.x; p < n; p += blockDim.x) {
-        const double v = (double)fr[p];
-        s += v * v;
-    }
-    s = block_sum(s, red);
-    if (threadIdx.x == 0)
-        *out = s;
-}
-
 cudaError_t launch_xcorr_shift(int dtype, const float* corr, const float* rowmax, const void* frames, long long fstride,
-                               const void* ref, const double* ref_sq, int nframes, int first_is_frame0,
-                               const Geometry& g, int* shifts, cudaStream_t st)
+                               const void* ref, const float* rowsq, int nsq, const float* refsq, double* ref_sq,
+                               int nframes, int first, const Geometry& g, int* shifts, cudaStream_t st)
 {
     // the correlation's FP32 error grows with the transforms' stages: log2(W H)
     // radix-2 stages; on the generic path log2 of the factors 2, 4 and 8
@@ -389,10 +395,10 @@ cudaError_t launch_xcorr_shift(int dtype, const float* corr, const float* rowmax
         for (int k = 0; k < g.pH.nf; ++k) stages += of(g.pH.fac[k]);
     }
     switch (dtype) {
-    case 0: xcorr_shift_kernel<uint8_t><<<nframes, kShiftThreads, 0, st>>>(corr, rowmax, (const uint8_t*)frames, fstride, (const uint8_t*)ref, ref_sq, first_is_frame0, g.W, logW, g.H, stages, shifts); note_launches(1); break;
-    case 1: xcorr_shift_kernel<uint16_t><<<nframes, kShiftThreads, 0, st>>>(corr, rowmax, (const uint16_t*)frames, fstride, (const uint16_t*)ref, ref_sq, first_is_frame0, g.W, logW, g.H, stages, shifts); note_launches(1); break;
-    case 2: xcorr_shift_kernel<float><<<nframes, kShiftThreads, 0, st>>>(corr, rowmax, (const float*)frames, fstride, (const float*)ref, ref_sq, first_is_frame0, g.W, logW, g.H, stages, shifts); note_launches(1); break;
-    default: xcorr_shift_kernel<double><<<nframes, kShiftThreads, 0, st>>>(corr, rowmax, (const double*)frames, fstride, (const double*)ref, ref_sq, first_is_frame0, g.W, logW, g.H, stages, shifts); note_launches(1); break;
+    case 0: xcorr_shift_kernel<uint8_t><<<nframes, kShiftThreads, 0, st>>>(corr, rowmax, (const uint8_t*)frames, fstride, (const uint8_t*)ref, rowsq, nsq, refsq, ref_sq, first, g.W, logW, g.H, stages, shifts); note_launches(1); break;
+    case 1: xcorr_shift_kernel<uint16_t><<<nframes, kShiftThreads, 0, st>>>(corr, rowmax, (const uint16_t*)frames, fstride, (const uint16_t*)ref, rowsq, nsq, refsq, ref_sq, first, g.W, logW, g.H, stages, shifts); note_launches(1); break;
+    case 2: xcorr_shift_kernel<float><<<nframes, kShiftThreads, 0, st>>>(corr, rowmax, (const float*)frames, fstride, (const float*)ref, rowsq, nsq, refsq, ref_sq, first, g.W, logW, g.H, stages, shifts); note_launches(1); break;
+    default: xcorr_shift_kernel<double><<<nframes, kShiftThreads, 0, st>>>(corr, rowmax, (const double*)frames, fstride, (const double*)ref, rowsq, nsq, refsq, ref_sq, first, g.W, logW, g.H, stages, shifts); note_launches(1); break;
     }
     return cudaGetLastError();
 }
@@ -401,7 +407,8 @@ cudaError_t launch_saa_add(int dtype, void* sum, const void* frames, long long f
                            int first_is_frame0, const int* shifts, const Geometry& g, cudaStream_t st)
 {
     const int n = g.W * g.H;
-    const int gx = (n + 255) / 256;
+    const int bs = dtype <= 1 ? 256 : 64;
+    const int gx = (n + bs - 1) / bs;
     // integer frames: frame groups of >= 32 frames, enough CTAs to fill a
     // 152-SM GPU about four deep
     constexpr int kTargetCtas = 4 * 152;
@@ -414,21 +421,10 @@ cudaError_t launch_saa_add(int dtype, void* sum, const void* frames, long long f
     const dim3 grid(gx, dtype <= 1 ? gy : 1);
     const size_t shm = sizeof(int2) * (size_t)(nframes > 0 ? (nframes + grid.y - 1) / grid.y + 1 : 1);
     switch (dtype) {
-    case 0: saa_add_kernel<uint8_t, unsigned long long><<<grid, 256, shm, st>>>((unsigned long long*)sum, (const uint8_t*)frames, fstride, nframes, first_is_frame0, shifts, g.W, g.H); note_launches(1); break;
-    case 1: saa_add_kernel<uint16_t, unsigned long long><<<grid, 256, shm, st>>>((unsigned long long*)sum, (const uint16_t*)frames, fstride, nframes, first_is_frame0, shifts, g.W, g.H); note_launches(1); break;
-    case 2: saa_add_kernel<float, double><<<grid, 256, shm, st>>>((double*)sum, (const float*)frames, fstride, nframes, first_is_frame0, shifts, g.W, g.H); note_launches(1); break;
-    default: saa_add_kernel<double, double><<<grid, 256, shm, st>>>((double*)sum, (const double*)frames, fstride, nframes, first_is_frame0, shifts, g.W, g.H); note_launches(1); break;
-    }
-    return cudaGetLastError();
-}
-
-cudaError_t launch_sumsq(int dtype, const void* frame, long long n, double* out, cudaStream_t st)
-{
-    switch (dtype) {
-    case 0: sumsq_kernel<uint8_t><<<1, 1024, 0, st>>>((const uint8_t*)frame, n, out); note_launches(1); break;
-    case 1: sumsq_kernel<uint16_t><<<1, 1024, 0, st>>>((const uint16_t*)frame, n, out); note_launches(1); break;
-    case 2: sumsq_kernel<float><<<1, 1024, 0, st>>>((const float*)frame, n, out); note_launches(1); break;
-    default: sumsq_kernel<double><<<1, 1024, 0, st>>>((const double*)frame, n, out); note_launches(1); break;
+    case 0: saa_add_kernel<uint8_t, unsigned long long, 8><<<grid, bs, shm, st>>>((unsigned long long*)sum, (const uint8_t*)frames, fstride, nframes, first_is_frame0, shifts, g.W, g.H); note_launches(1); break;
+    case 1: saa_add_kernel<uint16_t, unsigned long long, 8><<<grid, bs, shm, st>>>((unsigned long long*)sum, (const uint16_t*)frames, fstride, nframes, first_is_frame0, shifts, g.W, g.H); note_launches(1); break;
+    case 2: saa_add_kernel<float, double, 16><<<grid, bs, shm, st>>>((double*)sum, (const float*)frames, fstride, nframes, first_is_frame0, shifts, g.W, g.H); note_launches(1); break;
+    default: saa_add_kernel<double, double, 16><<<grid, bs, shm, st>>>((double*)sum, (const double*)frames, fstride, nframes, first_is_frame0, shifts, g.W, g.H); note_launches(1); break;
     }
     return cudaGetLastError();
 }

@@ -502,6 +502,7 @@ struct smip_stack {
     float2 *T = nullptr, *S = nullptr, *R = nullptr;
     float* corr = nullptr;
     float* rowmax = nullptr;      // per frame and row: the correlation's maximum
+    float* rowsq = nullptr;       // per frame and row block: the pixels' sum of squares
     float2* kscratch = nullptr;   // bispectrum kernel: partial sums of split tiles
     int* ktile_cnt = nullptr;     // bispectrum kernel: parts finished per split tile
     int* shifts = nullptr;        // all frames, int2
@@ -543,7 +544,7 @@ struct smip_stack {
             cudaStreamDestroy(cst);
         dfree(spec_staging);
         if (ref) cudaFree(ref);
-        dfree(ref_sq); dfree(Gt); dfree(T); dfree(S); dfree(R); dfree(corr); dfree(rowmax); dfree(shifts); dfree(err);
+        dfree(ref_sq); dfree(Gt); dfree(T); dfree(S); dfree(R); dfree(corr); dfree(rowmax); dfree(rowsq); dfree(shifts); dfree(err);
         dfree(kscratch); dfree(ktile_cnt);
         dfree(Z); dfree(pfull); dfree(maxbuf);
         free_gen_tw(&twW);
@@ -589,6 +590,7 @@ struct smip_stack {
         CUDA_TRY(cudaMalloc(&R, sizeof(float2) * half_elems()));
         CUDA_TRY(cudaMalloc(&corr, sizeof(float) * frame_elems() * Bf));
         CUDA_TRY(cudaMalloc(&rowmax, sizeof(float) * g.H * Bf));
+        CUDA_TRY(cudaMalloc(&rowsq, sizeof(float) * row_blocks(g) * Bf));
         CUDA_TRY(cudaMalloc(&ref_sq, sizeof(double)));
         CUDA_TRY(cudaMalloc(&err, sizeof(int)));
         CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(int), st));
@@ -694,41 +696,43 @@ struct smip_stack {
                 CUDA_TRY(cudaEventRecord(ev_copied[cur], cst));
                 CUDA_TRY(cudaStreamWaitEvent(q, ev_copied[cur], 0));
             }
-            if (first) {
+            if (first)
                 CUDA_TRY(cudaMemcpyAsync(ref, zc ? zc : staging, dtype_size(dtype) * fe, cudaMemcpyDefault, q));
-                CUDA_TRY(launch_sumsq(dtype, ref, (long long)fe, ref_sq, q));
-            }
+            // the reference's spectrum in a launch of its own where a line more
+            // in every chunk of frames would cost more than that launch (about 8 us)
+            const int ref_apart = first && n > 16 * fpc;
             if (g.generic) { // mixed-radix transforms (frame sizes other than powers of two in [16, 512])
                 if (zc) {
-                    CUDA_TRY(launch_gen_row_pass(dtype, zc, (long long)fe, n, g, Gt, twW.df, q, staging));
+                    CUDA_TRY(launch_gen_row_pass(dtype, zc, (long long)fe, n, g, Gt, rowsq, twW.df, q, staging));
                     CUDA_TRY(cudaEventRecord(ev_zc, q));
                     CUDA_TRY(cudaStreamWaitEvent(cst, ev_zc, 0));
                 } else {
-                    CUDA_TRY(launch_gen_row_pass(dtype, staging, (long long)fe, n, g, Gt, twW.df, q));
+                    CUDA_TRY(launch_gen_row_pass(dtype, staging, (long long)fe, n, g, Gt, rowsq, twW.df, q));
                 }
-                if (first)
-                    CUDA_TRY(launch_gen_col_pass(1, Gt, S, R, R, T, Ppart, 1, fpc, 0, g, twH.df, twH.f32, q));
-                CUDA_TRY(launch_gen_col_pass(0, Gt, S, R, nullptr, T, Ppart, n, fpc, first ? 1 : 0, g, twH.df, twH.f32,
+                if (ref_apart)
+                    CUDA_TRY(launch_gen_col_pass(Gt, S, R, T, Ppart, 1, fpc, 1, g, twH.df, twH.f32, q));
+                CUDA_TRY(launch_gen_col_pass(Gt, S, R, T, Ppart, n, fpc, first ? 1 + ref_apart : 0, g, twH.df, twH.f32,
                                              q));
                 CUDA_TRY(launch_power_reduce(P, Ppart, (n + fpc - 1) / fpc, g, q));
                 CUDA_TRY(launch_gen_xcorr_rows(T, corr, rowmax, n, g, twW.f32, q));
             } else {
                 if (zc) {
-                    CUDA_TRY(launch_row_pass(dtype, zc, (long long)fe, n, g, Gt, ctx->twdf, q, staging));
+                    CUDA_TRY(launch_row_pass(dtype, zc, (long long)fe, n, g, Gt, rowsq, ctx->twdf, q, staging));
                     CUDA_TRY(cudaEventRecord(ev_zc, q));
                     CUDA_TRY(cudaStreamWaitEvent(cst, ev_zc, 0));
                 } else {
-                    CUDA_TRY(launch_row_pass(dtype, staging, (long long)fe, n, g, Gt, ctx->twdf, q));
+                    CUDA_TRY(launch_row_pass(dtype, staging, (long long)fe, n, g, Gt, rowsq, ctx->twdf, q));
                 }
-                if (first)
-                    CUDA_TRY(launch_col_pass(1, Gt, S, R, R, T, Ppart, 1, fpc, 0, g, ctx->twdf, ctx->tw32, q));
-                CUDA_TRY(launch_col_pass(0, Gt, S, R, nullptr, T, Ppart, n, fpc, first ? 1 : 0, g, ctx->twdf,
+                if (ref_apart)
+                    CUDA_TRY(launch_col_pass(Gt, S, R, T, Ppart, 1, fpc, 1, g, ctx->twdf, ctx->tw32, q));
+                CUDA_TRY(launch_col_pass(Gt, S, R, T, Ppart, n, fpc, first ? 1 + ref_apart : 0, g, ctx->twdf,
                                          ctx->tw32, q));
                 CUDA_TRY(launch_power_reduce(P, Ppart, (n + fpc - 1) / fpc, g, q));
                 CUDA_TRY(launch_xcorr_rows(T, corr, rowmax, n, g, ctx->tw32, q));
             }
-            CUDA_TRY(launch_xcorr_shift(dtype, corr, rowmax, staging, (long long)fe, ref, ref_sq, n, first ? 1 : 0,
-                                        g, shifts + 2 * first_index, q));
+            CUDA_TRY(launch_xcorr_shift(dtype, corr, rowmax, staging, (long long)fe, ref, rowsq, row_blocks(g),
+                                        first ? rowsq : nullptr, ref_sq, n, first ? 1 : 0, g, shifts + 2 * first_index,
+                                        q));
             CUDA_TRY(launch_saa_add(dtype, sum, staging, (long long)fe, n, first ? 1 : 0, shifts + 2 * first_index, g, q));
         }
         if (!with_bispec)

@@ -299,6 +299,26 @@ __device__ void fft_passes(C* buf, int logn, int nl, int ls, const C* tw, int tw
     }
 }
 
+// The block's sum of v to *out (256 threads).  No barrier of its own is needed
+// after it: the next one orders the reads of the warps' sums.
+__device__ __forceinline__ void store_block_sum(float v, float* out)
+{
+    __shared__ float part[8];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+        v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0)
+        part[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float s = part[0];
+#pragma unroll
+        for (int i = 1; i < 8; ++i)
+            s += part[i];
+        *out = s;
+    }
+}
+
 // Copies the twiddle table (2^(twlog-1) entries) into shared memory.
 template <typename C>
 __device__ void load_twiddles(C* dst, const C* src, int twlog)

@@ -74,17 +74,21 @@ void set_error_message(const std::string& m);
 // All launchers are asynchronous on `st` and return cudaGetLastError().
 
 // frames (dtype) -> G'(a, y) = sum_x f(x,y) exp(+2 pi i a x / W), float-float,
-// stored [f][a][y].  dtype: 0 u8, 1 u16, 2 f32, 3 f64.  copy_out (optional,
-// device memory): the frames as read, same stride.
+// stored [f][a][y].  dtype: 0 u8, 1 u16, 2 f32, 3 f64.  rowsq[f][row_blocks(g)]:
+// FP32 sums of squares of the row blocks.  copy_out (optional, device memory):
+// the frames as read, same stride.
+int row_blocks(const Geometry& g);
 cudaError_t launch_row_pass(int dtype, const void* frames, long long frame_stride_elems, int nframes,
-                            const Geometry& g, dfc* Gt, const dfc* twdf, cudaStream_t st, void* copy_out = nullptr);
+                            const Geometry& g, dfc* Gt, float* rowsq, const dfc* twdf, cudaStream_t st,
+                            void* copy_out = nullptr);
 
-// Column pass.  mode 1: frame 0 only -> Rout (the reference spectrum).
-// mode 0: S[f][a][c] = F(-a, c - H/2), power partials, and the FP32 inverse
-// column FFT of conj(R)·F for the cross correlation into T[f][a][y].
-cudaError_t launch_col_pass(int mode, const dfc* Gt, float2* S, const float2* Rbuf, float2* Rout, float2* T,
-                            double* Ppart, int nframes, int frames_per_chunk, int skip_xcorr_frame0,
-                            const Geometry& g, const dfc* twdf, const float2* tw, cudaStream_t st);
+// Column pass: S[f][a][c] = F(-a, c - H/2), power partials, and the FP32 inverse
+// column FFT of conj(R)·F for the cross correlation into T[f][a][y].  first
+// non-zero: the batch's frame 0 is the reference, and its T is left out; 1: its
+// spectrum is formed and written to Rbuf, 2: it is there already.
+cudaError_t launch_col_pass(const dfc* Gt, float2* S, float2* Rbuf, float2* T, double* Ppart, int nframes,
+                            int frames_per_chunk, int first, const Geometry& g, const dfc* twdf, const float2* tw,
+                            cudaStream_t st);
 cudaError_t launch_power_reduce(double* P, const double* Ppart, int nchunks, const Geometry& g, cudaStream_t st);
 
 // Row pass of the correlation's inverse transform: corr[f][y][x] (float).
@@ -93,10 +97,13 @@ cudaError_t launch_xcorr_rows(const float2* T, float* corr, float* rowmax, int n
                               const float2* tw, cudaStream_t st);
 
 // Integer shift per frame: FP32 correlation peak, candidates re-scored exactly.
-// ref_sq: sum of squares of the reference frame (double, device).
+// rowsq, nsq: the row pass's sums of squares, nsq = row_blocks(g) per frame;
+// refsq: those of the reference, or null: *ref_sq (device) holds its sum.
+// first: frame 0 is the reference (refsq is given), *ref_sq is written.
 cudaError_t launch_xcorr_shift(int dtype, const float* corr, const float* rowmax, const void* frames,
-                               long long frame_stride_elems, const void* ref, const double* ref_sq, int nframes,
-                               int first_is_frame0, const Geometry& g, int* shifts, cudaStream_t st);
+                               long long frame_stride_elems, const void* ref, const float* rowsq, int nsq,
+                               const float* refsq, double* ref_sq, int nframes, int first, const Geometry& g,
+                               int* shifts, cudaStream_t st);
 
 // sum += |frames| shifted back by their shifts (Array2::shifted semantics);
 // the stack's frame 0 enters with its sign (smip-cli/main.cpp:266).
@@ -105,11 +112,11 @@ cudaError_t launch_saa_add(int dtype, void* sum, const void* frames, long long f
 
 // Mixed-radix counterparts of the three launchers above for the generic path
 // (k_fftg.cu); same inputs and outputs, twiddles from the stack's GenTw tables.
+int gen_row_blocks(const Geometry& g);
 cudaError_t launch_gen_row_pass(int dtype, const void* frames, long long fstride, int nframes, const Geometry& g,
-                                dfc* Gt, const dfc* twW, cudaStream_t st, void* copy_out = nullptr);
-cudaError_t launch_gen_col_pass(int mode, const dfc* Gt, float2* S, const float2* Rbuf, float2* Rout, float2* T,
-                                double* Ppart, int nframes, int fpc, int skip_xcorr_frame0, const Geometry& g,
-                                const dfc* twH, const float2* twH32, cudaStream_t st);
+                                dfc* Gt, float* rowsq, const dfc* twW, cudaStream_t st, void* copy_out = nullptr);
+cudaError_t launch_gen_col_pass(const dfc* Gt, float2* S, float2* Rbuf, float2* T, double* Ppart, int nframes, int fpc,
+                                int first, const Geometry& g, const dfc* twH, const float2* twH32, cudaStream_t st);
 cudaError_t launch_gen_xcorr_rows(const float2* T, float* corr, float* rowmax, int nframes, const Geometry& g,
                                   const float2* twW32, cudaStream_t st);
 // In-place FP64 transforms of nlines lines of length p.L (element stride es,
@@ -202,8 +209,5 @@ cudaError_t launch_power_full(const double* Phalf, double pnorm, const Geometry&
 cudaError_t launch_hann(double* out, int W, int H, double aperture, cudaStream_t st);
 // Array2<double>::shifted: out(x, y) = in(x - dx, y - dy), zero outside.
 cudaError_t launch_shifted(const double* in, double* out, int W, int H, int dx, int dy, cudaStream_t st);
-
-// Sum of squares of a frame (double), for the correlation error bound.
-cudaError_t launch_sumsq(int dtype, const void* frame, long long n, double* out, cudaStream_t st);
 
 } // namespace smip_gpu

@@ -46,15 +46,15 @@ constexpr int kMaxN = 256;                                   // largest ncols / 
 constexpr size_t kHalf = (size_t)(kMaxN / 2 + 1) * kMaxN;    // half-plane elements
 constexpr size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 constexpr size_t kOffGt = 0;                                             // 2 frames, float-float
-constexpr size_t kOffS = kOffGt + align256(2 * kHalf * sizeof(dfc));     // 1 frame
-constexpr size_t kOffT = kOffS + align256(kHalf * sizeof(float2));       // 1 frame
-constexpr size_t kOffR = kOffT + align256(kHalf * sizeof(float2));       // reference spectrum
+constexpr size_t kOffS = kOffGt + align256(2 * kHalf * sizeof(dfc));     // 2 frames
+constexpr size_t kOffT = kOffS + align256(2 * kHalf * sizeof(float2));   // 2 frames
+constexpr size_t kOffR = kOffT + align256(2 * kHalf * sizeof(float2));   // reference spectrum
 constexpr size_t kOffP = kOffR + align256(kHalf * sizeof(float2));       // power partials
 constexpr size_t kOffC = kOffP + align256(kHalf * sizeof(double));       // correlation
 constexpr size_t kOffM = kOffC + align256((size_t)kMaxN * kMaxN * sizeof(float)); // row maxima
-constexpr size_t kOffQ = kOffM + align256((size_t)kMaxN * sizeof(float));          // sum of squares
+constexpr size_t kOffQ = kOffM + align256((size_t)kMaxN * sizeof(float));          // sums of squares, 2 frames
 constexpr int kTw = 1 << (kTwLog - 1);
-constexpr size_t kOffTw = kOffQ + 256;                                   // FP32 twiddles
+constexpr size_t kOffTw = kOffQ + align256(2 * (size_t)kMaxN * sizeof(float));     // FP32 twiddles
 constexpr size_t kOffTwDf = kOffTw + align256(kTw * sizeof(float2));     // float-float twiddles
 constexpr size_t kOffWarm = kOffTwDf + align256(kTw * sizeof(dfc));     // warm-up frame (16 x 16 doubles, zero)
 constexpr size_t kWarmN = 16;
@@ -145,17 +145,26 @@ cudaError_t run_shift(unsigned char* base, const double* ref, const double* fram
     double* Pp = reinterpret_cast<double*>(base + kOffP);
     float* corr = reinterpret_cast<float*>(base + kOffC);
     float* rowmax = reinterpret_cast<float*>(base + kOffM);
-    double* refsq = reinterpret_cast<double*>(base + kOffQ);
+    float* rowsq = reinterpret_cast<float*>(base + kOffQ);
+    const int nsq = row_blocks(g);
     const float2* tw = reinterpret_cast<const float2*>(base + kOffTw);
     const dfc* twdf = reinterpret_cast<const dfc*>(base + kOffTwDf);
     const long long n = (long long)ncols * nrows;
-    cudaError_t e = launch_sumsq(SMIP_F64, ref, n, refsq, st);
-    if (e == cudaSuccess) e = launch_row_pass(SMIP_F64, ref, n, 1, g, Gt, twdf, st);
-    if (e == cudaSuccess) e = launch_row_pass(SMIP_F64, frame, n, 1, g, Gt + half, twdf, st);
-    if (e == cudaSuccess) e = launch_col_pass(1, Gt, S, R, R, T, Pp, 1, 16, 0, g, twdf, tw, st);
-    if (e == cudaSuccess) e = launch_col_pass(0, Gt + half, S, R, nullptr, T, Pp, 1, 16, 0, g, twdf, tw, st);
-    if (e == cudaSuccess) e = launch_xcorr_rows(T, corr, rowmax, 1, g, tw, st);
-    if (e == cudaSuccess) e = launch_xcorr_shift(SMIP_F64, corr, rowmax, frame, n, ref, refsq, 1, 0, g, shift, st);
+    // reference and frame as a batch of two: two launches to the spectra and the
+    // correlation's columns, two to the shift.  The frames are one stride apart
+    // when their distance is a whole number of pixels.
+    cudaError_t e;
+    const long long apart = reinterpret_cast<const char*>(frame) - reinterpret_cast<const char*>(ref);
+    if (apart % (long long)sizeof(double) == 0) {
+        e = launch_row_pass(SMIP_F64, ref, apart / (long long)sizeof(double), 2, g, Gt, rowsq, twdf, st);
+    } else {
+        e = launch_row_pass(SMIP_F64, ref, n, 1, g, Gt, rowsq, twdf, st);
+        if (e == cudaSuccess) e = launch_row_pass(SMIP_F64, frame, n, 1, g, Gt + half, rowsq + nsq, twdf, st);
+    }
+    if (e == cudaSuccess) e = launch_col_pass(Gt, S, R, T, Pp, 2, 16, 1, g, twdf, tw, st);
+    if (e == cudaSuccess) e = launch_xcorr_rows(T + half, corr, rowmax, 1, g, tw, st);
+    if (e == cudaSuccess)
+        e = launch_xcorr_shift(SMIP_F64, corr, rowmax, frame, n, ref, rowsq + nsq, nsq, rowsq, nullptr, 1, 0, g, shift, st);
     return e;
 }
 
