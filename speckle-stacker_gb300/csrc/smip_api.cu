@@ -101,6 +101,38 @@ struct DeviceCtx {
 std::mutex g_ctx_mu;
 std::map<int, DeviceCtx> g_ctx;
 
+// Device error words.  They lie in page-locked host memory that the kernels
+// write through (record_error, on a failure only), so that a result call reads
+// one after its own wait instead of copying it: a copy of four bytes and its
+// wait cost about 10 us, four times a job.  Pages are made as they are needed
+// and kept; a stack takes a word and gives it back.
+std::mutex g_err_mu;
+std::vector<int*> g_err_free;
+
+int take_err_word(int** out)
+{
+    std::lock_guard<std::mutex> lk(g_err_mu);
+    if (g_err_free.empty()) {
+        int* page = nullptr;
+        constexpr int kStep = 64 / (int)sizeof(int), kWords = 64; // a cache line each
+        CUDA_TRY(cudaHostAlloc(&page, (size_t)kWords * kStep * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped));
+        for (int i = 0; i < kWords; ++i)
+            g_err_free.push_back(page + i * kStep);
+    }
+    *out = g_err_free.back();
+    g_err_free.pop_back();
+    **out = 0;
+    return SMIP_OK;
+}
+
+void give_err_word(int* w)
+{
+    if (!w)
+        return;
+    std::lock_guard<std::mutex> lk(g_err_mu);
+    g_err_free.push_back(w);
+}
+
 int device_ctx(int dev, DeviceCtx** out)
 {
     std::lock_guard<std::mutex> lk(g_ctx_mu);
@@ -435,16 +467,20 @@ struct Reco {
     }
 };
 
-int check_dev_err(int* err_dev, cudaStream_t st)
+int dev_err_status(int e)
 {
-    int e = 0;
-    CUDA_TRY(cudaMemcpyAsync(&e, err_dev, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
     if (e == SMIP_DEV_ERR_TIMEOUT)
         return fail(SMIP_E_TIMEOUT, "a bounded device wait expired; results of the affected batch are incomplete");
     if (e == SMIP_DEV_ERR_OUT_OF_RANGE)
         return fail(SMIP_E_OUT_OF_RANGE, "Bispectrum: element address out of bounds (get_element would throw)");
     return SMIP_OK;
+}
+
+// Waits for the stream and reports what its kernels recorded.
+int check_dev_err(const int* err, cudaStream_t st)
+{
+    CUDA_TRY(cudaStreamSynchronize(st));
+    return dev_err_status(*reinterpret_cast<const volatile int*>(err));
 }
 
 } // namespace
@@ -475,6 +511,9 @@ struct smip_stack {
     double k2_frames = 0.0;
     std::vector<int> ev_frames;
     // device buffers
+    // everything that a reset zeroes, in one allocation: B, C, P, sum, ktile_cnt
+    unsigned char* zeroed = nullptr;
+    size_t zeroed_bytes = 0;
     float2 *B = nullptr, *C = nullptr, *Bn = nullptr;
     double* P = nullptr;
     double* Ppart = nullptr;
@@ -530,8 +569,8 @@ struct smip_stack {
         }
         if (ev_reco) cudaEventDestroy(ev_reco);
         if (ev_dep) cudaEventDestroy(ev_dep);
-        dfree(B); dfree(C); dfree(Bn); dfree(P); dfree(Ppart);
-        if (sum) cudaFree(sum);
+        dfree(zeroed);
+        dfree(Bn); dfree(Ppart);
         if (cst)
             cudaStreamSynchronize(cst);
         for (int i = 0; i < 2; ++i) {
@@ -544,8 +583,8 @@ struct smip_stack {
             cudaStreamDestroy(cst);
         dfree(spec_staging);
         if (ref) cudaFree(ref);
-        dfree(ref_sq); dfree(Gt); dfree(T); dfree(S); dfree(R); dfree(corr); dfree(rowmax); dfree(rowsq); dfree(shifts); dfree(err);
-        dfree(kscratch); dfree(ktile_cnt);
+        dfree(ref_sq); dfree(Gt); dfree(T); dfree(S); dfree(R); dfree(corr); dfree(rowmax); dfree(rowsq); dfree(shifts);
+        dfree(kscratch);
         dfree(Z); dfree(pfull); dfree(maxbuf);
         free_gen_tw(&twW);
         free_gen_tw(&twH);
@@ -555,6 +594,7 @@ struct smip_stack {
         }
         if (own_stream && st)
             cudaStreamDestroy(st);
+        give_err_word(err);
     }
 
     size_t frame_elems() const { return (size_t)g.W * g.H; }
@@ -563,16 +603,18 @@ struct smip_stack {
     int alloc()
     {
         const size_t bs = (size_t)g.base_size;
-        CUDA_TRY(cudaMalloc(&B, sizeof(float2) * bs));
-        CUDA_TRY(cudaMalloc(&C, sizeof(float2) * bs));
-        CUDA_TRY(cudaMemsetAsync(B, 0, sizeof(float2) * bs, st));
-        CUDA_TRY(cudaMemsetAsync(C, 0, sizeof(float2) * bs, st));
-        CUDA_TRY(cudaMalloc(&P, sizeof(double) * half_elems()));
-        CUDA_TRY(cudaMemsetAsync(P, 0, sizeof(double) * half_elems(), st));
+        auto up = [](size_t n) { return (n + 255) / 256 * 256; };
+        const size_t nb = up(sizeof(float2) * bs), np = up(sizeof(double) * half_elems()), ns = up(8 * frame_elems());
+        zeroed_bytes = 2 * nb + np + ns + up(sizeof(int) * bispec_tile_counters(ctx->num_sms));
+        CUDA_TRY(cudaMalloc(&zeroed, zeroed_bytes));
+        CUDA_TRY(cudaMemsetAsync(zeroed, 0, zeroed_bytes, st));
+        B = reinterpret_cast<float2*>(zeroed);
+        C = reinterpret_cast<float2*>(zeroed + nb);
+        P = reinterpret_cast<double*>(zeroed + 2 * nb);
+        sum = zeroed + 2 * nb + np;
+        ktile_cnt = reinterpret_cast<int*>(zeroed + 2 * nb + np + ns);
         const int nchunks = (Bf + fpc - 1) / fpc;
         CUDA_TRY(cudaMalloc(&Ppart, sizeof(double) * half_elems() * nchunks));
-        CUDA_TRY(cudaMalloc(&sum, 8 * frame_elems()));
-        CUDA_TRY(cudaMemsetAsync(sum, 0, 8 * frame_elems(), st));
         CUDA_TRY(cudaMalloc(&Gt, sizeof(dfc) * half_elems() * Bf));
         CUDA_TRY(cudaMalloc(&T, sizeof(float2) * half_elems() * Bf));
         CUDA_TRY(cudaMalloc(&S, sizeof(float2) * (size_t)g.hw * g.Hs * Bf));
@@ -592,16 +634,14 @@ struct smip_stack {
         CUDA_TRY(cudaMalloc(&rowmax, sizeof(float) * g.H * Bf));
         CUDA_TRY(cudaMalloc(&rowsq, sizeof(float) * row_blocks(g) * Bf));
         CUDA_TRY(cudaMalloc(&ref_sq, sizeof(double)));
-        CUDA_TRY(cudaMalloc(&err, sizeof(int)));
-        CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(int), st));
+        if (int rc = take_err_word(&err))
+            return rc;
         // Everything a job needs is allocated here, with the stack, so that a
         // pooled stack serves further jobs without allocating: an allocation
         // (and a free, which synchronises the device) in the middle of
         // serving stalls the request loop until the GPU drains.
         CUDA_TRY(cudaMalloc(&ref, 8 * frame_elems()));
         CUDA_TRY(cudaMalloc(&kscratch, bispec_scratch_bytes(ctx->num_sms)));
-        CUDA_TRY(cudaMalloc(&ktile_cnt, sizeof(int) * bispec_tile_counters(ctx->num_sms)));
-        CUDA_TRY(cudaMemsetAsync(ktile_cnt, 0, sizeof(int) * bispec_tile_counters(ctx->num_sms), st));
         return ensure_shift_cap(kShiftCap0);
     }
 
@@ -1018,14 +1058,9 @@ extern "C" int smip_stack_reset(smip_stack_t s)
         CUDA_TRY(cudaStreamSynchronize(s->cst));
     if ((rc = s->collect_timing()))
         return rc;
-    const size_t bs = (size_t)s->g.base_size;
-    CUDA_TRY(cudaMemsetAsync(s->B, 0, sizeof(float2) * bs, s->st));
-    CUDA_TRY(cudaMemsetAsync(s->C, 0, sizeof(float2) * bs, s->st));
-    CUDA_TRY(cudaMemsetAsync(s->P, 0, sizeof(double) * s->half_elems(), s->st));
-    CUDA_TRY(cudaMemsetAsync(s->sum, 0, 8 * s->frame_elems(), s->st));
-    CUDA_TRY(cudaMemsetAsync(s->err, 0, sizeof(int), s->st));
-    if (s->ktile_cnt) // a launch that stopped early (timeout) may leave parts counted
-        CUDA_TRY(cudaMemsetAsync(s->ktile_cnt, 0, sizeof(int) * bispec_tile_counters(s->ctx->num_sms), s->st));
+    *s->err = 0; // the stream is idle
+    // (the tile counters too: a launch that stopped early may leave parts counted)
+    CUDA_TRY(cudaMemsetAsync(s->zeroed, 0, s->zeroed_bytes, s->st));
     s->nframes = 0;
     s->pending = 0;
     s->has_ref = false;
@@ -1246,22 +1281,28 @@ extern "C" int smip_diag_bounded_wait(int device, double timeout_s)
         return fail(SMIP_E_INVALID_ARGUMENT, "timeout must be in (0, 10] s");
     CUDA_TRY(cudaSetDevice(device));
     cudaStream_t st = nullptr;
-    int* buf = nullptr; // [0] device error word, [1] the flag nothing sets
-    CUDA_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+    int *err = nullptr, *never = nullptr; // the error word; the flag nothing sets
+    if (int rc = take_err_word(&err))
+        return rc;
     int rc = SMIP_OK;
-    cudaError_t e = cudaMalloc(&buf, 2 * sizeof(int));
+    cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
     if (e == cudaSuccess)
-        e = cudaMemsetAsync(buf, 0, 2 * sizeof(int), st);
+        e = cudaMalloc(&never, sizeof(int));
     if (e == cudaSuccess)
-        e = launch_bounded_wait_probe(buf, buf + 1, timeout_s, st);
+        e = cudaMemsetAsync(never, 0, sizeof(int), st);
+    if (e == cudaSuccess)
+        e = launch_bounded_wait_probe(err, never, timeout_s, st);
     if (e != cudaSuccess)
         rc = fail(SMIP_E_CUDA, cudaGetErrorString(e));
     else
-        rc = check_dev_err(buf, st); // SMIP_E_TIMEOUT, as after any expired wait
-    cudaStreamSynchronize(st);
-    if (buf)
-        cudaFree(buf);
-    cudaStreamDestroy(st);
+        rc = check_dev_err(err, st); // SMIP_E_TIMEOUT, as after any expired wait
+    if (st) {
+        cudaStreamSynchronize(st);
+        cudaStreamDestroy(st);
+    }
+    if (never)
+        cudaFree(never);
+    give_err_word(err);
     return rc;
 }
 
@@ -1764,12 +1805,12 @@ extern "C" int smip_reconstruct_phases(int device, const float* bispec, long xsi
     {
         Reco reco;
         reco.g = g;
-        if (cudaMalloc(&Bd, sizeof(float2) * g.base_size) != cudaSuccess || cudaMalloc(&err, sizeof(int)) != cudaSuccess)
+        if (cudaMalloc(&Bd, sizeof(float2) * g.base_size) != cudaSuccess)
             rc = fail(SMIP_E_NO_MEMORY, "device allocation failed");
+        if (!rc)
+            rc = take_err_word(&err);
         if (!rc && cudaMemcpyAsync(Bd, bispec, sizeof(float2) * g.base_size, cudaMemcpyHostToDevice, st) != cudaSuccess)
             rc = fail(SMIP_E_CUDA, "bispectrum upload failed");
-        if (!rc && cudaMemsetAsync(err, 0, sizeof(int), st) != cudaSuccess)
-            rc = fail(SMIP_E_CUDA, "memset failed");
         if (!rc)
             rc = reco.run(Bd, R, err, st);
         if (!rc)
@@ -1779,7 +1820,7 @@ extern "C" int smip_reconstruct_phases(int device, const float* bispec, long xsi
         cudaStreamSynchronize(st);
     }
     if (Bd) cudaFree(Bd);
-    if (err) cudaFree(err);
+    give_err_word(err);
     cudaStreamDestroy(st);
     return rc;
 }
