@@ -329,15 +329,17 @@ __global__ void __launch_bounds__(32 * kPlanWarps) spiral_plan_kernel(const Reco
 // cluster).
 //   warp 0 of rank 0 (the serial warp) runs the visits in order;
 //   the writer, on another sub-partition, copies what the serial warp found
-//     into the phase map in global memory and publishes the progress to every
-//     CTA;
-//   summing warps form, for visit q, the share of the non-recent pairs once
-//     the progress has reached q - kRecoLag, resolve the recent pairs' members
-//     that lie outside the lag, and post both into slot q mod kRing of rank 0;
-//   gathering warps of rank 0 wait for the other CTAs' posts (st.async, whose
-//     completion the slot's mbarrier counts: a plain store and a release at
-//     cluster scope held the summing warp for 2,200 cycles a visit), add a
-//     visit's parts and set the tag that the serial warp looks at.
+//     into the phase map in global memory and publishes the progress, first to
+//     its own CTA, whose warps need no release at cluster scope;
+//   loading warps bring visit q's recent pairs into slot q mod kRing of rank 0
+//     once the progress has reached q - kRecoLag, with the members that lie
+//     outside the lag;
+//   summing warps form the share of the non-recent pairs, at the same progress,
+//     and post it to that slot (st.async, whose completion the slot's mbarrier
+//     counts: a plain store and a release at cluster scope held the summing warp
+//     for 2,200 cycles a visit);
+//   gathering warps wait for both, add a visit's parts and set the tag that the
+//     serial warp looks at.
 // In a cluster rank 0 sums nothing; in a lone CTA the summing warps are those
 // of the other three SM sub-partitions, so that the serial warp keeps the
 // issue slots of its own.
@@ -345,28 +347,42 @@ __global__ void __launch_bounds__(32 * kPlanWarps) spiral_plan_kernel(const Reco
 // What a visit must wait for is the phase of the visit just before it.  The
 // serial warp therefore does everything else of visit q + 1 while the chain of
 // visit q runs: the terms of the pairs of age >= 2, and their butterfly sum
-// over the lanes, of which lane 0 keeps the sibling sum that it receives at
-// each level.  Lane 0 holds the one pair of age 1: its term, five additions of
-// those sibling sums (bit for bit the butterfly's result), the float-float
-// addition to the share and the phase are the chain, with no shuffle, branch
-// or memory access between two visits.  Visits that are not "fast" (two pairs
-// of age 1, or more than 32 recent pairs: near the origin, 2 % of the visits
-// at 256 x 256) form their sum at once, as 32 or 64 terms.
+// over the lanes (real parts in the lower half warp, imaginary parts in the
+// upper, after its first level), of which lanes 0 and 16 keep the sibling sums
+// that they receive.  Every lane forms the first pair's term, the only one of
+// age 1: that, five additions of the sibling sums (bit for bit the butterfly's
+// result), the float-float addition to the share, one exchange between lanes 0
+// and 16 and the phase are the chain.  Visits that are "wide" (two pairs of age
+// 1, more than 32 recent pairs, or a point visited within the lag: near the
+// origin, 2 % of the visits at 256 x 256) form their sum at once, as 32 or 64
+// terms.
+//
+// A share waits for its u's, which come from L2 (the other SMs write them).  The
+// plan row of a visit does not depend on the chain: a bulk copy brings it into
+// the summing CTA's shared memory before the visit may be summed, so that up to
+// 20 gathers a lane are in flight with 2 registers each (10 with the row's
+// elements in registers beside them: 1,800 cycles a batch; now 3,300 for 19 or 20
+// words).
 //
 // The phase map is kept centred with De / 2 points of padding and holds NaN
 // where there is no phase, so that a pair's u is one address and needs no
 // bounds or flag test: a product with an unflagged or outside point is NaN.
 // Every wait is bounded; on a timeout the walk stops and the error is recorded.
 //
-// Bound by latency: the chain and the early part of one visit, issued by one
-// warp, take 306 cycles on an idle SM; a visit of the walk takes about 450
-// (2,000 before: 256 x 256, d = 32, R = 128 in 14.4 ms instead of 56.9, and
-// 512 x 512, d = 48, R = 200 in 34.7 ms instead of 153.7).
+// Bound by the serial warp, which waits for instructions as much as for the
+// chain (200 cycles): a visit takes 458 / 442 / 428 cycles at depths 24 / 32 / 48
+// (495 / 472 / 465 with the recent pairs loaded by the summing warps, the whole
+// butterfly in one step and addresses formed in the loop; 2,000 with everything
+// in the serial warp).  128 x 128, d = 24, R = 48 in 2.04 ms (2.34, 7.8), 256 x
+// 256, d = 32, R = 128 in 13.7 (15.3, 58.2), 512 x 512, d = 48, R = 200 in 34.9
+// (41.5, 163), normalisation and plan included.  A sum of the recent pairs by age instead
+// of by slot needs no butterfly at all and takes 330 cycles, but rounds
+// otherwise: the phases then differ by up to 5e-7.
 constexpr int kRing = 64;
 constexpr int kMaxParts = 6;
 constexpr int kStep = 4;                 // visits between two looks of the serial warp at the other warps
 constexpr int kGroups = kRing / kStep;
-constexpr int kSkip = 0, kFast = 1, kWide = 2; // ctl.z: how the serial warp treats a visit
+constexpr int kRowWords = 40;            // words of a plan row that a summing warp of a cluster keeps in shared memory
 constexpr unsigned long long kRecoWaitNs = 2000000000ull;
 static_assert(kRing > kRecoLag + 8, "ring slots outlive the lag and the serial warp's look-ahead");
 
@@ -400,23 +416,51 @@ __device__ __forceinline__ float2 ld_stream(const float2* p)
     return v;
 }
 
-static size_t walk_smem(int nslots) { return sizeof(float4) * (nslots + kRing * kRecentMax + kRing + 1) + sizeof(unsigned) * kRing * kRecentMax; }
+// Dynamic shared memory, offsets in bytes.  What the serial warp reads and writes
+// lies at constant offsets, so that a slot's number is its only address
+// arithmetic.  Ranks above 0 keep their plan rows there instead.  v's phase and
+// map offset are at the end.
+constexpr int kShareAt = 0;                      // float4 [kRing]: sum of the non-recent pairs (re hi, lo, im hi, lo)
+constexpr int kCtlAt = kShareAt + 16 * kRing;    // float4 [kRing]: phase the point already has (or NaN), kCtl bits, number of those pairs (far below 0: the point has its phase, or can have none)
+constexpr int kSumAt = kCtlAt + 16 * kRing;      // float4 [kRing]: sums of the last visits, for the writer
+constexpr int kPhaseAt = kSumAt + 16 * kRing;    // float4 [kRing]: phases of the last visits, pairs of a point that got its phase
+constexpr int kHeadAt = kPhaseAt + 16 * kRing;   // float4 [kRing]: the first recent pair: phasor, offsets of u's and v's phase
+constexpr int kPairAt = kHeadAt + 16 * kRing;    // float4 [kRing][kRecentMax]: phasor, the member outside the lag
+constexpr int kPlaceAt = kPairAt + 16 * kRing * kRecentMax; // uint2 [kRing][kRecentMax]: offsets of u's and v's phase
+constexpr int kRingBytes = kPlaceAt + 8 * kRing * kRecentMax;
+// kCtl: age of the point's own last visit | two sets of pairs << 8 | the first pair's u, v is the last phase << 9, << 10
+__host__ __device__ constexpr size_t box_bytes(int nslots) { return (size_t)nslots * (sizeof(float2) + sizeof(int)); }
+// words of a visit's longest part, and whether they fit
+__host__ __device__ __forceinline__ int part_words(int De, int nwords) { return (nwords + share_parts(De, nwords) - 1) / share_parts(De, nwords); }
+static size_t walk_smem(int De, int nslots, bool multi)
+{
+    size_t most = (size_t)kRingBytes; // of any depth up to De: the jobs of a launch may differ
+    for (int d = 0; multi && d <= De; d += 2) {
+        const int pw = part_words(d, ((d + 1) * (d + 1) + 31) / 32);
+        const size_t rows = pw <= kRowWords ? (size_t)pw * 256 * (kRecoThreads / 32) : 0;
+        most = rows > most ? rows : most;
+    }
+    return box_bytes(nslots) + most;
+}
 
 // CTAs per job: as few as keep the serial warp busy, because jobs that share
-// the GPU need the other SMs.  Cycles a visit with 1 / 2 / 4 CTAs: 583 / 493 /
-// 490 at depth 24, 708 / 595 / 475 at depth 32 (a lone CTA's summing warps have
-// three sub-partitions); at depth 48 seven summing CTAs keep up (461).
+// the GPU need the other SMs.  Cycles a visit with 2 / 4 / 8 CTAs: 459 / 456 /
+// 455 at depth 24, 528 / 440 / 435 at depth 32; with 4 / 8: 479 / 428 at depth 48.
+// (A lone CTA, where no cluster can be placed: 1,054 at depth 24, 1,241 at 32.)
 static int walk_ctas(int De) { return De < 28 ? 2 : (De < kPartsDepth ? 4 : 8); }
 
 template <bool MULTI> // a cluster of CTAs per job, or one CTA
 __global__ void __launch_bounds__(kRecoThreads, 1) phase_walk_kernel(const RecoJob* __restrict__ jobs)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
-    __shared__ float4 shr[kMaxParts + 1][kRing]; // share of the non-recent pairs: re hi, lo, im hi, lo; row kMaxParts: the parts' sum
-    __shared__ int shn[kMaxParts + 1][kRing];
-    __shared__ int tag_s[kMaxParts + 1][kRing];  // visit + 1 whose part has landed; row kMaxParts: all of it, gathered
-    __shared__ float4 ctl[kRing];            // phase the point already has (or NaN), kind of visit, kc | two sets << 8
-    __shared__ float4 res_s[kRing + 1];      // sums of the last visits, for the writer (+ a place for what nobody reads)
+    __shared__ float4 shr[kMaxParts][kRing];     // a part's sum over the non-recent pairs: re hi, lo, im hi, lo
+    __shared__ int shn[kMaxParts][kRing];        // its number of pairs
+    __shared__ float4 shc[kRing];                // number of pairs of part 0, the phase that the point already has
+    __shared__ int tag_s[kMaxParts][kRing];      // visit + 1 whose part has landed (lone CTA)
+    __shared__ int gtag[kRing];                  // 2 (visit + 1) + wide: the visit is ready for the serial warp
+    __shared__ int lhead[kRing];                 // kCtl bits of the visit's first pair
+    __shared__ int ltag[kRing];                  // visit + 1 whose recent pairs have been loaded
+    __shared__ __align__(8) uint64_t row_bar[kRecoThreads / 32]; // a summing warp's plan row has arrived
     __shared__ __align__(8) uint64_t ring_bar[kRing];   // cluster: visit q's parts have landed in slot q mod kRing
     __shared__ __align__(8) uint64_t done_bar[kGroups]; // the serial warp has finished kStep more visits
     __shared__ int progress;   // visits whose phases are published (a copy in every CTA)
@@ -425,21 +469,27 @@ __global__ void __launch_bounds__(kRecoThreads, 1) phase_walk_kernel(const RecoJ
     const RecoJob J = jobs[blockIdx.x / ncta];
     const int W = J.W, H = J.H, De = J.De, e = De / 2;
     const int nside = De + 1, nv = nside * nside, nwords = (nv + 31) / 32, nslots = nwords * 32;
-    const int nparts = share_parts(De, nwords), share_row = nparts > 1 ? kMaxParts : 0;
-    const int tag_row = MULTI ? kMaxParts : share_row; // what tells the serial warp that a visit has been posted
+    const int nparts = share_parts(De, nwords);
     const int PW = W + De;
-    float4* vt = reinterpret_cast<float4*>(smraw); // [nslots] phase of v, map offset of v
-    float4* ent = vt + nslots;                     // [kRing][kRecentMax] phasor, the member outside the lag (rank 0)
-    float4* res_p = ent + kRing * kRecentMax;      // [kRing + 1] phases of the last visits, pairs of a point that got its phase
-    // where a recent pair's u and v lie, in units of 8 bytes from ent (a last
-    // phase's slot, or the posted member): u | v << 16, bits 14 and 30: the
-    // phase of the visit just before, bit 31: the phasor is out of range
-    unsigned* ecode = reinterpret_cast<unsigned*>(res_p + kRing + 1); // [kRing][kRecentMax]
+    unsigned box_at; // the same in every CTA of the cluster
+    asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(box_at));
+    box_at -= (unsigned)box_bytes(nslots);
+    float2* vt = reinterpret_cast<float2*>(smraw + box_at); // [nslots] phase of v
+    int* voff = reinterpret_cast<int*>(vt + nslots);        // [nslots] map offset of v
+    float2* rows = reinterpret_cast<float2*>(smraw);        // ranks above 0: a plan row per warp
+    float4* share = reinterpret_cast<float4*>(smraw + kShareAt);
+    float4* ctl = reinterpret_cast<float4*>(smraw + kCtlAt);
+    float4* res_s = reinterpret_cast<float4*>(smraw + kSumAt);
+    float4* res_p = reinterpret_cast<float4*>(smraw + kPhaseAt);
+    float4* head = reinterpret_cast<float4*>(smraw + kHeadAt);
+    float4* ent = reinterpret_cast<float4*>(smraw + kPairAt);
+    uint2* place = reinterpret_cast<uint2*>(smraw + kPlaceAt);
+    auto phase_at = [&](unsigned off) { return *reinterpret_cast<const float2*>(smraw + off); };
     const float nanf_ = __uint_as_float(kUnusable);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int t = threadIdx.x; t < nslots; t += blockDim.x) {
         const int vx = -e + t % nside, vy = -e + t / nside;
-        float4 v = make_float4(nanf_, nanf_, __int_as_float(t < nv ? vy * PW + vx : 0), 0.f);
+        float2 v = make_float2(nanf_, nanf_);
         if (t < nv && abs(vx) + abs(vy) <= 1) { // seeds (phasereco.h:42-54)
             v.x = 1.f;
             v.y = vx < 0 || vy < 0 ? -0.f : 0.f;
@@ -451,13 +501,25 @@ __global__ void __launch_bounds__(kRecoThreads, 1) phase_walk_kernel(const RecoJ
             }
         }
         vt[t] = v;
+        voff[t] = t < nv ? vy * PW + vx : 0;
     }
-    for (int i = threadIdx.x; i < (kMaxParts + 1) * kRing; i += blockDim.x)
+    for (int i = threadIdx.x; i < kMaxParts * kRing; i += blockDim.x)
         (&tag_s[0][0])[i] = 0;
-    // a slot is read before its first pairs are posted (a visit with nothing
-    // to sum posts none): its codes must be places within ent at all times
-    for (int i = threadIdx.x; i < kRing * kRecentMax; i += blockDim.x)
-        ecode[i] = 0u;
+    for (int i = threadIdx.x; i < kRing; i += blockDim.x)
+        ltag[i] = gtag[i] = 0;
+    // a slot may be read before anything is posted to it: its offsets are
+    // places of phases at all times
+    if (rank == 0) {
+        for (int i = threadIdx.x; i < kRing * kRecentMax; i += blockDim.x) {
+            place[i] = make_uint2(kPhaseAt, kPhaseAt);
+            ent[i] = make_float4(nanf_, nanf_, nanf_, nanf_);
+        }
+        for (int i = threadIdx.x; i < kRing; i += blockDim.x) {
+            share[i] = res_s[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            ctl[i] = res_p[i] = make_float4(nanf_, nanf_, 0.f, 0.f);
+            head[i] = make_float4(nanf_, nanf_, __uint_as_float(kPhaseAt), __uint_as_float(kPhaseAt));
+        }
+    }
     if (threadIdx.x == 0) {
         progress = 0;
         abort_walk = 0;
@@ -465,6 +527,8 @@ __global__ void __launch_bounds__(kRecoThreads, 1) phase_walk_kernel(const RecoJ
             mbar_init(&ring_bar[i], nparts); // an arrival per part
         for (int i = 0; i < kGroups; ++i)
             mbar_init(&done_bar[i], 1);
+        for (int i = 0; i < kRecoThreads / 32; ++i)
+            mbar_init(&row_bar[i], 1);
         fence_mbar_init();
     }
     __threadfence(); // the seeds in the map
@@ -513,53 +577,37 @@ __global__ void __launch_bounds__(kRecoThreads, 1) phase_walk_kernel(const RecoJ
             record_error(J.err, SMIP_DEV_ERR_OUT_OF_RANGE);
     };
 
-    const bool on_rank0 = !MULTI || rank == 0;
-    if (on_rank0 && warp == 0) {
+    // which warp does what (a nibble each): 0 the serial warp, 1 the writer,
+    // 2.. loading, 6.. gathering, 14 summing, 15 nothing.  In a cluster rank 0
+    // sums nothing; the serial warp's sub-partition (warp % 4) is its own in a
+    // cluster, and free of summing warps in a lone CTA.
+    constexpr unsigned long long kRoles = MULTI ? 0xFB5F432FA91F8760ull : 0xEEE2EEE6EEE1EEE0ull;
+    constexpr int kLoaders = MULTI ? 4 : 1, kGatherers = MULTI ? 6 : 1;
+    const int role = MULTI && rank != 0 ? 14 : (int)(kRoles >> (4 * warp)) & 15;
+    // the map: other SMs write it in a cluster (read from L2), this SM in a lone CTA
+    auto map_at = [&](long long i) { return MULTI ? __ldcg(J.pmap + i) : *(J.pmap + i); };
+    // this CTA's copy of the progress has reached v
+    auto reached = [&](int v) { return __all_sync(0xffffffffu, wait_until([&] { return ld_acquire_cta(&progress) >= v; }, 20u) ? 1 : 0); };
+    if (role == 0) {
         // ------------------------------------------------ serial warp
-        struct Vis { // a visit as posted
-            float2 bh; // phasor
-            unsigned c; // where its members lie
-            float4 k;  // ctl
-        };
-        const float2* mem = reinterpret_cast<const float2*>(ent);
-        auto load_vis = [&](int q, Vis& v) {
-            const int s = q & (kRing - 1);
-            v.bh = mem[2 * (s * kRecentMax + lane)];
-            v.c = ecode[s * kRecentMax + lane];
-            v.k = ctl[s];
-        };
-        auto members = [&](unsigned c, float2& U, float2& V) {
-            U = mem[c & 0x3fffu];
-            V = mem[(c >> 16) & 0x3fffu];
-        };
         auto term = [&](float2 U, float2 V, float2 bh, float2& p, float& r) {
             p = pair_product(U, V, bh.x, bh.y);
             const float n2 = norm2(p);
             r = rsqrt_ftz(n2);
             return !isnan(n2);
         };
-        // a point's phase from its float-float sum and number of pairs; FP64
-        // values are formed after the walk.  A sum above the limit has a
-        // normal square.
-        auto phase_from = [&](float4 sum, int cnt) {
-            const float s2 = norm2(make_float2(sum.x, sum.z));
-            const float lim = 2.220446049250313e-16f * (float)cnt;
-            const float r = rsqrt_ftz(s2);
-            float2 pf = s2 > lim * lim ? make_float2(sum.x * r, sum.z * r) : make_float2(0.f, 0.f);
-            pf.x = cnt > 0 ? pf.x : nanf_; // no pair: no phase
-            pf.y = cnt > 0 ? pf.y : nanf_;
-            return pf;
-        };
-        // visits [q, q + kStep) (or up to the last) are ready: relaxed polls and
-        // one fence of this CTA's scope, which costs nothing (a fence of the
-        // cluster's takes 300 cycles: the gathering warps do those)
-        auto ready = [&](int q) {
-            const int v = q + (lane & (kStep - 1)) < J.nvisits ? q + (lane & (kStep - 1)) : J.nvisits - 1;
-            const volatile int* tag = &tag_s[tag_row][v & (kRing - 1)];
+        // visits [q, q + kStep) (or up to the last) are ready, and which of them
+        // are wide: relaxed polls and one fence of this CTA's scope, which costs
+        // nothing (a fence of the cluster's takes 300 cycles)
+        auto ready = [&](int q, unsigned& wide) {
+            const int at = q + (lane & (kStep - 1)), v = at < J.nvisits ? at : J.nvisits - 1;
+            const volatile int* tag = &gtag[v & (kRing - 1)];
             unsigned long long t0 = 0;
             for (int n = 1;; ++n) {
-                if (__all_sync(0xffffffffu, *tag == v + 1)) {
+                const int t = *tag;
+                if (__all_sync(0xffffffffu, t >> 1 == v + 1)) {
                     __threadfence_block();
+                    wide = __ballot_sync(0xffffffffu, lane < kStep && (t & 1) && at < J.nvisits);
                     return true;
                 }
                 if (n & 63)
@@ -576,342 +624,426 @@ __global__ void __launch_bounds__(kRecoThreads, 1) phase_walk_kernel(const RecoJ
             }
         };
         const int nqs = (J.nvisits + kStep - 1) / kStep * kStep; // the writer leaves out what lies past the last visit
-        Vis v0, v1, v2; // visits q, q + 1, q + 2
-        // what is known of visit q before the phase of visit q - 1
-        float2 eU, eV;      // members (lane 0: one of them is that phase)
-        float sR[5], sI[5]; // the sibling sums of the butterfly's levels
-        int ecnt;           // pairs but lane 0's, and the share's
-        float4 esum;        // share of the non-recent pairs
-        auto early = [&](int q, const Vis& v) {
-            esum = shr[share_row][q & (kRing - 1)];
-            ecnt = shn[share_row][q & (kRing - 1)];
+        const bool imag = lane >= 16; // lanes 0 and 16 form the real and the imaginary part
+        float2 last = make_float2(nanf_, nanf_);
+        uint2 lc = {}, hc = {};            // places of visit q + 1's members: the lane's pair, the first pair
+        float2 hU = {}, hV = {}, hb = {};  // visit q's first pair
+        float sib0 = 0.f, level = 0.f;     // visit q's recent pairs in the butterfly: the first pair's sibling, and its first level
+        float en = 0.f;                    // its recent pairs but the first
+        // what can be known of visit q before the phase of visit q - 1: the terms
+        // of the lanes' pairs (the first's is left out) and the first level of
+        // their butterfly sum, from which on the lower lanes hold real parts and the
+        // upper ones imaginary parts.  The other levels run beside the next step's
+        // chain: all of them in one step would make it as long as they are.
+        auto early = [&](float2 U, float2 V, float2 b) {
             float2 p;
             float r;
-            const bool ok = term(eU, eV, v.bh, p, r);
-            float x = ok ? fmaf(p.x, r, 0.f) : 0.f, y = ok ? fmaf(p.y, r, 0.f) : 0.f;
-            ecnt += __popc(__ballot_sync(0xffffffffu, ok) & ~1u);
+            const bool ok = term(U, V, b, p, r);
+            const float x = ok ? fmaf(p.x, r, 0.f) : 0.f, y = ok ? fmaf(p.y, r, 0.f) : 0.f;
+            en = (float)__popc(__ballot_sync(0xffffffffu, ok) & ~1u);
+            float a = imag ? y : x;
+            const float o = __shfl_xor_sync(0xffffffffu, imag ? x : y, 16);
+            sib0 = imag ? a : o;
+            level = __fadd_rn(a, o);
+        };
+        // The sum of a visit from its recent pairs' (lanes 0 and 16) and its
+        // share, its phase and what is kept of it.  FP64 values are formed after
+        // the walk; a sum above the limit has a normal square; a point without
+        // any pair has no phase.
+        auto finish = [&](float part, float2 sh, float4 ct, float cnt, float2& kept) {
+            const float s = __fadd_rn(sh.x, part), bb = __fsub_rn(s, sh.x);
+            const float e = __fadd_rn(__fadd_rn(__fsub_rn(sh.x, __fsub_rn(s, bb)), __fsub_rn(part, bb)), sh.y);
+            kept = make_float2(s, e);
+            const float h = __fadd_rn(s, e);
+            const float2 f = make_float2(__shfl_sync(0xffffffffu, h, 0), __shfl_sync(0xffffffffu, h, 16));
+            const float s2 = norm2(f), r = rsqrt_ftz(s2), lim = 2.220446049250313e-16f * cnt;
+            const bool has = cnt > 0.f, normal = has && s2 > lim * lim;
+            float2 now = make_float2(has ? 0.f : ct.x, has ? 0.f : ct.y);
+            now.x = normal ? f.x * r : now.x;
+            now.y = normal ? f.y * r : now.y;
+            return now;
+        };
+        auto share_of = [&](int s) { return *reinterpret_cast<const float2*>(smraw + kShareAt + 16 * s + (imag ? 8 : 0)); };
+        auto keep = [&](int s, float cnt, float2 kept) {
+            res_p[s] = make_float4(last.x, last.y, cnt, 0.f); // the same in every lane
+            if ((lane & 15) == 0)
+                *reinterpret_cast<float2*>(smraw + kSumAt + 16 * s + (imag ? 8 : 0)) = kept;
+            __syncwarp();
+        };
+        // visit q; the chain (the first pair's term, five additions, the share,
+        // the phase) and the early part of visit q + 1 overlap
+        auto step = [&](int q) {
+            const int s = q & (kRing - 1), s1 = (q + 1) & (kRing - 1), s2 = (q + 2) & (kRing - 1);
+            const float2 sh = share_of(s);
+            const float4 ct = ctl[s];
+            const float2 nU = phase_at(lc.x), nV = phase_at(lc.y), nhU = phase_at(hc.x), nhV = phase_at(hc.y);
+            const float4* ne = &ent[s1 * kRecentMax + lane];
+            const float2 nb = make_float2(ne->x, ne->y), nhb = make_float2(head[s1].x, head[s1].y);
+            lc = place[s2 * kRecentMax + lane];
+            hc = make_uint2(__float_as_uint(head[s2].z), __float_as_uint(head[s2].w));
+            const int bits = __float_as_int(ct.z);
+            const bool lu = bits & (1 << 9), lv = bits & (1 << 10);
+            // sibling sums on the first pair's way down the butterfly (lanes 0, 16)
+            float sib[5] = { sib0 };
 #pragma unroll
-            for (int l = 0; l < 5; ++l) {
-                sR[l] = __shfl_xor_sync(0xffffffffu, x, 16 >> l);
-                sI[l] = __shfl_xor_sync(0xffffffffu, y, 16 >> l);
-                x = __fadd_rn(x, sR[l]);
-                y = __fadd_rn(y, sI[l]);
+            for (int l = 1; l < 5; ++l) {
+                sib[l] = __shfl_xor_sync(0xffffffffu, level, 16 >> l);
+                level = __fadd_rn(level, sib[l]);
             }
+            float2 p, kept;
+            float r;
+            const bool ok = term(make_float2(lu ? last.x : hU.x, lu ? last.y : hU.y),
+                                 make_float2(lv ? last.x : hV.x, lv ? last.y : hV.y), hb, p, r);
+            float a = ok ? fmaf(imag ? p.y : p.x, r, 0.f) : 0.f;
+#pragma unroll
+            for (int l = 0; l < 5; ++l)
+                a = __fadd_rn(a, sib[l]);
+            const float cnt = ct.w + en + (ok ? 1.f : 0.f);
+            early(nU, nV, nb);
+            last = finish(a, sh, ct, cnt, kept);
+            keep(s, cnt, kept);
+            hU = nhU;
+            hV = nhV;
+            hb = nhb;
         };
-        float2 last = make_float2(nanf_, nanf_);
-        // every lane stores a visit's result, lane 0 (whose result it is) to
-        // its slot, the others to a slot that nobody reads
-        const int smul = lane == 0 ? 1 : 0, sadd = lane == 0 ? 0 : kRing;
-        auto store = [&](int q, float4 sum, int cnt) {
-            const int s = (q & (kRing - 1)) * smul + sadd;
-            res_p[s] = make_float4(last.x, last.y, __int_as_float(cnt), 0.f);
-            res_s[s] = sum;
+        // a visit with up to 64 recent pairs, several of age 1, or whose point may
+        // have got its phase within the lag: all terms now, the phases up to the
+        // last lie in their slots
+        auto wide_step = [&](int q) {
+            const int s = q & (kRing - 1), s1 = (q + 1) & (kRing - 1), s2 = (q + 2) & (kRing - 1);
+            const float2 sh = share_of(s);
+            const float4 ct = ctl[s];
+            const int bits = __float_as_int(ct.z), kc = bits & 63;
+            const bool two = bits & (1 << 8);
+            const uint2 ca = place[s * kRecentMax + lane], cb = place[s * kRecentMax + 32 + lane];
+            const float4 ba = ent[s * kRecentMax + lane], bb = ent[s * kRecentMax + 32 + lane];
+            const float2 Ua = phase_at(ca.x), Va = phase_at(ca.y), Ub = phase_at(cb.x), Vb = phase_at(cb.y);
+            const float4 own = res_p[(q - kc) & (kRing - 1)];
+            float2 pa, pb, kept;
+            float ra, rb;
+            const bool oka = term(Ua, Va, make_float2(ba.x, ba.y), pa, ra);
+            const bool okb = term(Ub, Vb, make_float2(bb.x, bb.y), pb, rb) && two;
+            float sr = oka ? fmaf(pa.x, ra, 0.f) : 0.f, si = oka ? fmaf(pa.y, ra, 0.f) : 0.f;
+            sr = okb ? fmaf(pb.x, rb, sr) : sr;
+            si = okb ? fmaf(pb.y, rb, si) : si;
+            float cnt = ct.w + (float)(__popc(__ballot_sync(0xffffffffu, oka)) + __popc(__ballot_sync(0xffffffffu, okb)));
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                sr = __fadd_rn(sr, __shfl_xor_sync(0xffffffffu, sr, o));
+                si = __fadd_rn(si, __shfl_xor_sync(0xffffffffu, si, o));
+            }
+            float2 now = finish(imag ? si : sr, sh, ct, cnt, kept);
+            if (kc && !isnan(own.x)) { // its point, visited within the lag, has its phase
+                now = make_float2(own.x, own.y);
+                cnt = 0.f;
+            } else if (oor_any && q < J.nvisits) {
+                check_oor(__float_as_uint(ba.x) == kOorBits, Ua, Va);
+                check_oor(two && __float_as_uint(bb.x) == kOorBits, Ub, Vb);
+            }
+            const float4* ne = &ent[s1 * kRecentMax + lane];
+            early(phase_at(lc.x), phase_at(lc.y), make_float2(ne->x, ne->y));
+            hU = phase_at(hc.x);
+            hV = phase_at(hc.y);
+            hb = make_float2(head[s1].x, head[s1].y);
+            lc = place[s2 * kRecentMax + lane];
+            hc = make_uint2(__float_as_uint(head[s2].z), __float_as_uint(head[s2].w));
+            last = now;
+            keep(s, cnt, kept);
         };
-        bool go = ready(0) && ready(2);
+        unsigned wide = 0u, more = 0u; // wide visits from q on
+        bool go = ready(0, wide) && ready(2, more);
+        wide = (wide & 3u) | more << 2;
         if (go) {
-            load_vis(0, v0);
-            load_vis(1, v1);
-            members(v0.c, eU, eV);
-            early(0, v0);
+            const float4* e0 = &ent[lane];
+            const uint2 c0 = place[lane];
+            early(phase_at(c0.x), phase_at(c0.y), make_float2(e0->x, e0->y));
+            hb = make_float2(head[0].x, head[0].y);
+            hU = phase_at(__float_as_uint(head[0].z));
+            hV = phase_at(__float_as_uint(head[0].w));
+            lc = place[kRecentMax + lane];
+            hc = make_uint2(__float_as_uint(head[1].z), __float_as_uint(head[1].w));
         }
         for (int q = 0; go && q < nqs;) {
-            if (__float_as_int(v0.k.z) != kWide) {
-                // The loop's body is one block without branches, for the fast
-                // visits and those with nothing to do, so that the chain of
-                // visit q (lane 0) and the early part of visit q + 1 overlap.
-                do {
-                    load_vis(q + 2, v2); // used one visit later
-                    const int kind = __float_as_int(v0.k.z);
-                    float2 nU, nV;
-                    members(v1.c, nU, nV);
-                    const bool lu = v0.c & 0x4000u, lv = v0.c & 0x40000000u;
-                    const float2 U = make_float2(lu ? last.x : eU.x, lu ? last.y : eU.y);
-                    const float2 V = make_float2(lv ? last.x : eV.x, lv ? last.y : eV.y);
-                    float2 p;
-                    float r;
-                    const bool ok = term(U, V, v0.bh, p, r);
-                    float x = ok ? fmaf(p.x, r, 0.f) : 0.f, y = ok ? fmaf(p.y, r, 0.f) : 0.f;
-    #pragma unroll
-                    for (int l = 0; l < 5; ++l) {
-                        x = __fadd_rn(x, sR[l]);
-                        y = __fadd_rn(y, sI[l]);
-                    }
-                    int cnt = ecnt + (ok ? 1 : 0);
-                    float4 sum = esum;
-                    ff_add(sum.x, sum.y, x, 0.f);
-                    ff_add(sum.z, sum.w, y, 0.f);
-                    last = phase_from(sum, cnt);
-                    cnt = kind == kFast ? cnt : 0;
-                    last.x = kind == kFast ? last.x : v0.k.x;
-                    last.y = kind == kFast ? last.y : v0.k.y;
-                    eU = nU;
-                    eV = nV;
-                    early(q + 1, v1);
-                    store(q, sum, cnt);
-                    __syncwarp();
-                    v0 = v1;
-                    v1 = v2;
-                    ++q;
-                } while (((q & (kStep - 1)) != 0) & (__float_as_int(v0.k.z) != kWide));
-            } else { // all terms now: the phases up to the last lie in their slots
-                load_vis(q + 2, v2);
-                const int s = q & (kRing - 1), kc = __float_as_int(v0.k.w) & 63;
-                const bool two = (__float_as_int(v0.k.w) >> 8) != 0;
-                float2 Ua, Va, Ub, Vb, pa, pb;
-                float ra, rb;
-                members(v0.c, Ua, Va);
-                const unsigned cb = ecode[s * kRecentMax + 32 + lane];
-                const float2 bb = mem[2 * (s * kRecentMax + 32 + lane)];
-                members(cb, Ub, Vb);
-                const float4 own = res_p[(q - kc) & (kRing - 1)];
-                float4 sum = shr[share_row][s];
-                int cnt = shn[share_row][s];
-                const bool oka = term(Ua, Va, v0.bh, pa, ra);
-                const bool okb = term(Ub, Vb, bb, pb, rb) && two;
-                float sr = oka ? fmaf(pa.x, ra, 0.f) : 0.f, si = oka ? fmaf(pa.y, ra, 0.f) : 0.f;
-                sr = okb ? fmaf(pb.x, rb, sr) : sr;
-                si = okb ? fmaf(pb.y, rb, si) : si;
-                cnt += __popc(__ballot_sync(0xffffffffu, oka)) + __popc(__ballot_sync(0xffffffffu, okb));
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    sr = __fadd_rn(sr, __shfl_xor_sync(0xffffffffu, sr, o));
-                    si = __fadd_rn(si, __shfl_xor_sync(0xffffffffu, si, o));
+            // a loop of one block without branches; unrolled it was slower (493
+            // cycles a visit instead of 428 at depth 48), as with both forms in
+            // one loop (568): the warp waits for instructions
+            if ((wide & ((1u << kStep) - 1u)) == 0u) {
+#pragma unroll 1
+                for (int k = 0; k < kStep; ++k)
+                    step(q + k);
+            } else {
+#pragma unroll 1
+                for (int k = 0; k < kStep; ++k) {
+                    if ((wide >> k) & 1u)
+                        wide_step(q + k);
+                    else
+                        step(q + k);
                 }
-                ff_add(sum.x, sum.y, sr, 0.f);
-                ff_add(sum.z, sum.w, si, 0.f);
-                last = phase_from(sum, cnt);
-                if (kc && !isnan(own.x)) { // its point, visited within the lag, has its phase
-                    last = make_float2(own.x, own.y);
-                    cnt = 0;
-                } else if (oor_any && q < J.nvisits) {
-                    check_oor(v0.c >> 31, Ua, Va);
-                    check_oor(two && (cb >> 31), Ub, Vb);
-                }
-                members(v1.c, eU, eV);
-                early(q + 1, v1);
-                store(q, sum, cnt);
-                __syncwarp();
-                v0 = v1;
-                v1 = v2;
-                ++q;
             }
-            if ((q & (kStep - 1)) == 0) { // tell the writer, look ahead
-                if (lane == 0)
-                    mbar_arrive(&done_bar[(q / kStep - 1) & (kGroups - 1)]);
-                go = ready(q + 2);
-            }
+            q += kStep;
+            wide >>= kStep;
+            // tell the writer, look ahead
+            if (lane == 0)
+                mbar_arrive(&done_bar[(q / kStep - 1) & (kGroups - 1)]);
+            go = ready(q + 2, more);
+            wide |= more << 2;
         }
-    } else if (on_rank0 && warp == (MULTI ? 5 : 4)) {
+    } else if (role == 1) {
         // ------------------------------------------------------ writer
         const int ngroups = (J.nvisits + kStep - 1) / kStep;
         for (int g = 0; g < ngroups;) {
             // groups of kStep visits, as many as are done (up to 32 visits)
+            const int q = kStep * g + lane, s = q & (kRing - 1);
+            int4 m = make_int4(-1, 0, 0, -1);
+            if (q < J.nvisits)
+                m = J.meta[q];
             auto is_done = [&](int h) { return mbar_test_wait(&done_bar[h & (kGroups - 1)], (uint32_t)(h / kGroups) & 1u); };
             if (!__all_sync(0xffffffffu, wait_until([&] { return is_done(g); }, 20u) ? 1 : 0))
                 break;
             const unsigned m8 = __ballot_sync(0xffffffffu, lane < 32 / kStep && g + lane < ngroups && is_done(g + lane)) | 1u;
             const int n = __ffs(~m8) - 1;
-            const int q = kStep * g + lane, s = q & (kRing - 1);
+            float4 rp = make_float4(0.f, 0.f, 0.f, 0.f), rs = rp;
             if (lane < kStep * n && q < J.nvisits) {
-                const float4 rp = res_p[s];
-                const int cnt = __float_as_int(rp.z);
-                if (cnt > 0) { // a point got its phase
-                    const int4 m = J.meta[q];
-                    const float2 pf = make_float2(rp.x, rp.y);
-                    J.pmap[m.x] = pf;
-                    J.sums[m.y] = res_s[s];
-                    J.cnt[m.y] = cnt;
-                    if (m.w >= 0) {
-                        if constexpr (MULTI) {
-                            for (uint32_t c = 0; c < ncta; ++c)
-                                dsmem_st_f2(dsmem_addr(&vt[m.w], c), pf);
-                        } else {
-                            *reinterpret_cast<float2*>(&vt[m.w]) = pf;
-                        }
-                    }
-                }
+                rp = res_p[s];
+                rs = res_s[s];
+            }
+            const int cnt = (int)rp.z;
+            const float2 pf = make_float2(rp.x, rp.y);
+            if (cnt > 0) { // a point got its phase
+                J.pmap[m.x] = pf;
+                if (m.w >= 0)
+                    vt[m.w] = pf;
             }
             g += n;
             __syncwarp();
-            // release: the stores above come before it for whoever acquires it
+            // release: the stores above come before it for whoever acquires it,
+            // first in this CTA, whose warps wait for nothing else
+            if (lane == 0)
+                st_release_cta(&progress, kStep * g);
             if constexpr (MULTI) {
-                if (lane < (int)ncta)
+                if (cnt > 0 && m.w >= 0)
+                    for (uint32_t c = 1; c < ncta; ++c)
+                        dsmem_st_f2(dsmem_addr(&vt[m.w], c), pf);
+                __syncwarp();
+                if (lane > 0 && lane < (int)ncta)
                     dsmem_st_release(dsmem_addr(&progress, lane), kStep * g);
-            } else {
-                if (lane == 0)
-                    st_release_cta(&progress, kStep * g);
+            }
+            if (cnt > 0) { // read after the walk only
+                J.sums[m.y] = rs;
+                J.cnt[m.y] = cnt;
             }
             __syncwarp();
         }
-    } else if (on_rank0 && tag_row == kMaxParts && (MULTI ? warp < 4 || warp == 6 : warp == 8 || warp == 12)) {
-        // gathering warps: a visit's parts, in part order, and the other CTAs'
-        // data on to the serial warp
-        const int c = MULTI ? (warp == 6 ? 3 : warp - 1) : warp / 4 - 2, ncomb = MULTI ? 4 : 2;
-        for (int q = c; q < J.nvisits; q += ncomb) {
+    } else if (role < 6) {
+        // ------- loading warps: a visit's recent pairs, with their members
+        // outside the lag, whose phases are final
+        int4 nm = make_int4(-1, 0, 0, -1);
+        uint4 na = make_uint4(kUnusable, kUnusable, 0u, 0u), nb = na;
+        auto fetch = [&](int q) { // the list of a point that is not runnable was never written
+            if (q < J.nvisits) {
+                nm = J.meta[q];
+                na = J.rec[(long long)q * kRecentMax + lane];
+                nb = J.rec[(long long)q * kRecentMax + 32 + lane];
+            }
+        };
+        fetch(role - 2);
+        for (int q = role - 2; q < J.nvisits; q += kLoaders) {
+            const int4 m = nm;
+            const uint4 ra = na, rb = nb;
             const int s = q & (kRing - 1);
-            const volatile int* tag = &tag_s[lane < nparts ? lane : 0][s];
-            if (!__all_sync(0xffffffffu, wait_until([&] {
-                                return MULTI ? mbar_try_wait_cluster(&ring_bar[s], (uint32_t)(q / kRing) & 1u) : *tag == q + 1;
-                            }, MULTI ? 0u : 20u) ? 1 : 0))
+            fetch(q + kLoaders);
+            if (!reached(q - kRecoLag))
                 break;
-            __threadfence_block();
-            if (nparts > 1) {
-                float4 sum = shr[0][s];
-                int n = shn[0][s];
-                for (int pp = 1; pp < nparts; ++pp) {
-                    const float4 op = shr[pp][s];
-                    ff_add(sum.x, sum.y, op.x, op.y);
-                    ff_add(sum.z, sum.w, op.z, op.w);
-                    n += shn[pp][s];
+            auto post = [&](int at, uint4 r) {
+                const int t = r.z & 0x1fff, ku = (r.z >> 13) & 63, kv = (r.z >> 19) & 63;
+                float2 x = vt[t]; // v, unless u is the one outside the lag
+                if (!ku && kv)
+                    x = map_at((long long)m.x - voff[t]);
+                ent[s * kRecentMax + at] = make_float4(__uint_as_float(r.x), __uint_as_float(r.y), x.x, x.y);
+                const unsigned own = kPairAt + 16u * (s * kRecentMax + at) + 8u;
+                const uint2 c = make_uint2(ku ? kPhaseAt + 16u * ((q - ku) & (kRing - 1)) : own,
+                                           kv ? kPhaseAt + 16u * ((q - kv) & (kRing - 1)) : own);
+                place[s * kRecentMax + at] = c;
+                if (at == 0) {
+                    head[s] = make_float4(__uint_as_float(r.x), __uint_as_float(r.y), __uint_as_float(c.x), __uint_as_float(c.y));
+                    lhead[s] = (ku == 1 ? 1 << 9 : 0) | (kv == 1 ? 1 << 10 : 0);
                 }
-                if (lane == 0) {
-                    shr[kMaxParts][s] = sum;
-                    shn[kMaxParts][s] = n;
-                }
+            };
+            if ((m.z >> 17) & 1) {
+                post(lane, ra);
+                if ((m.z & 255) > 32)
+                    post(lane + 32, rb);
             }
             __syncwarp();
             if (lane == 0)
-                st_release_cta(&tag_s[kMaxParts][s], q + 1);
+                st_release_cta(&ltag[s], q + 1);
         }
-    } else if (MULTI ? rank != 0 : (warp & 3) != 0) {
-        // ------------------------------------------- non-recent shares
-        const int nsum = MULTI ? (int)(ncta - 1) * (kRecoThreads / 32) : kRecoThreads / 32 * 3 / 4;
-        const int g = MULTI ? (int)(rank - 1) * (kRecoThreads / 32) + warp : (warp >> 2) * 3 + (warp & 3) - 1;
-        const long long nitems = (long long)J.nvisits * nparts; // (visit, part), visits in order
-        // A part's words in nbat batches of nbw or nbw - 1: the pair slots per
-        // lane in flight, as many as the registers hold (18 spilled).
-        constexpr int kB = 10;
-        const int longest = (nwords + nparts - 1) / nparts;
-        const int nbat = (longest + kB - 1) / kB, nbw = (longest + nbat - 1) / nbat;
-        for (long long it = g; it < nitems; it += nsum) {
-            const int q = (int)(it / nparts), part = (int)(it - (long long)q * nparts);
-            const int wb = part * nwords / nparts, we = (part + 1) * nwords / nparts;
-            const int4 m = J.meta[q];
-            const float2* prow = J.plan + (long long)q * nslots + lane;
-            uint4 ra = make_uint4(kUnusable, kUnusable, 0u, 0u), rb = ra;
-            const int rc = m.z & 255, kc = (m.z >> 8) & 63;
-            const bool run = (m.z >> 17) & 1;
-            if (part == 0 && run) {
-                ra = J.rec[(long long)q * kRecentMax + lane];
-                if (rc > 32)
-                    rb = J.rec[(long long)q * kRecentMax + 32 + lane];
+    } else if (role < 14) {
+        // gathering warps: a visit's parts, in part order, and what its point has
+        int4 nm = make_int4(-1, 0, 0, -1);
+        if (role - 6 < J.nvisits)
+            nm = J.meta[role - 6];
+        for (int q = role - 6; q < J.nvisits; q += kGatherers) {
+            const int s = q & (kRing - 1);
+            const int4 m = nm;
+            if (q + kGatherers < J.nvisits)
+                nm = J.meta[q + kGatherers];
+            const volatile int* tag = &tag_s[lane < nparts ? lane : 0][s];
+            const volatile int* lt = &ltag[s];
+            if (!__all_sync(0xffffffffu, wait_until([&] {
+                                return MULTI ? mbar_try_wait_cluster(&ring_bar[s], (uint32_t)(q / kRing) & 1u) : *tag == q + 1;
+                            }, MULTI ? 0u : 20u) && wait_until([&] { return *lt == q + 1; }, 20u) ? 1 : 0))
+                break;
+            __threadfence_block();
+            float4 sum = shr[0][s];
+            const float4 c = shc[s];
+            int n = __float_as_int(c.x);
+            for (int pp = 1; pp < nparts; ++pp) {
+                const float4 op = shr[pp][s];
+                ff_add(sum.x, sum.y, op.x, op.y);
+                ff_add(sum.z, sum.w, op.z, op.w);
+                n += shn[pp][s];
             }
-            if (lane == 0 && it + nsum < nitems) { // the next item's plan row on its way into L2
-                const long long nx = it + nsum;
-                const int nq = (int)(nx / nparts), np = (int)(nx - (long long)nq * nparts);
-                const int b = np * nwords / nparts, l = (np + 1) * nwords / nparts - b;
-                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(J.plan + (long long)nq * nslots + 32 * b),
-                             "r"(l * 32 * (int)sizeof(float2))
+            if (lane == 0) {
+                // a point outside the map, a seed, or one that has its phase: nothing to sum
+                const int rc = m.z & 255, kc = (m.z >> 8) & 63;
+                const bool skip = !((m.z >> 17) & 1) || (kc == 0 && !isnan(c.y));
+                const bool wide = !skip && (!((m.z >> 16) & 1) || oor_any);
+                share[s] = sum;
+                ctl[s] = make_float4(c.y, c.z, __int_as_float(kc | (rc > 32 ? 1 << 8 : 0) | (skip ? 0 : lhead[s])), skip ? -1e6f : (float)n);
+                st_release_cta(&gtag[s], 2 * (q + 1) + (wide ? 1 : 0));
+            }
+            __syncwarp();
+        }
+    } else if (role == 14) {
+        // ------------------------------------------- non-recent shares
+        // Warp g takes part g % nparts of the visits g / nparts, + at_once, ..
+        const int nsum = MULTI ? (int)(ncta - 1) * (kRecoThreads / 32) : kRecoThreads / 32 * 3 / 4;
+        const int g = MULTI ? warp * (int)(ncta - 1) + (int)(rank - 1) : (warp >> 2) * 3 + (warp & 3) - 1;
+        const int at_once = nsum / nparts, part = g % nparts, q0 = g < at_once * nparts ? g / nparts : J.nvisits;
+        const int wb = part * nwords / nparts, we = (part + 1) * nwords / nparts;
+        // In a cluster a visit's plan row comes into shared memory before the
+        // visit may be summed, and only the gathers of u stand between the
+        // progress and the sum: kB of them a lane in flight (2 registers each).
+        constexpr int kB = 20, kBDirect = 10;
+        const int nbat = (we - wb + kB - 1) / kB, nbw = (we - wb + nbat - 1) / nbat; // batches, words of one
+        const bool staged = MULTI && part_words(De, nwords) <= kRowWords;
+        float2* row = rows + warp * part_words(De, nwords) * 32;
+        auto is_run = [&](const int4& m) { return ((m.z >> 17) & 1) != 0; };
+        bool flying = false; // a copy of a row is on its way, or has not been waited for
+        uint32_t phase = 0u;
+        auto stage = [&](int q, const int4& m) {
+            flying = staged && is_run(m);
+            if (flying && lane == 0) {
+                const uint32_t bytes = (uint32_t)(we - wb) * 256u;
+                mbar_arrive_expect_tx(&row_bar[warp], bytes);
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(row)),
+                             "l"(J.plan + (long long)q * nslots + 32 * wb), "r"(bytes), "r"(smem_u32(&row_bar[warp]))
                              : "memory");
+            }
+        };
+        int4 nm = make_int4(-1, 0, 0, -1); // the next visit's meta, and the phase that its point has so far
+        float nx = nanf_;
+        if (q0 < J.nvisits) {
+            nm = J.meta[q0];
+            stage(q0, nm);
+        }
+        for (int q = q0; q < J.nvisits; q += at_once) {
+            const int4 m = nm;
+            const int kc = (m.z >> 8) & 63;
+            // a point outside the map, a seed, or one that has its phase: nothing
+            // to sum (a phase once set stays; a point that has none yet is looked
+            // at again below)
+            bool skip = !is_run(m) || (kc == 0 && !isnan(nx));
+            if (q + at_once < J.nvisits) {
+                nm = J.meta[q + at_once];
+                if (lane == 0) // the next visit's plan row on its way into L2
+                    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(J.plan + (long long)(q + at_once) * nslots + 32 * wb),
+                                 "r"((we - wb) * 32 * (int)sizeof(float2))
+                                 : "memory");
             }
             if (!__all_sync(0xffffffffu, wait_until([&] {
                                 const int pr = MULTI ? dsmem_ld_acquire(dsmem_addr(&progress, rank)) : ld_acquire_cta(&progress);
                                 return pr >= q - kRecoLag;
                             }, 20u) ? 1 : 0))
                 break;
-            // the map: other SMs write it in a cluster (read from L2), this SM in a lone CTA
-            auto map_at = [&](long long i) { return MULTI ? __ldcg(J.pmap + i) : *(J.pmap + i); };
-            float2 cur = make_float2(nanf_, nanf_);
+            if (oor_any && !skip && kc == 0) // the errors of a point that has its phase do not count
+                skip = !isnan(map_at(m.x).x);
+            float2 cur = make_float2(nanf_, nanf_); // waited for at the end
             if (m.x >= 0)
                 cur = map_at(m.x);
-            // a point outside the map, a seed, or one that has its phase: nothing to sum
-            const bool skip = !run || (kc == 0 && !isnan(cur.x));
-            const int s = q & (kRing - 1);
-            const uint32_t bar = MULTI ? dsmem_addr(&ring_bar[s], 0) : 0u;
-            auto put4 = [&](float4* p, float4 v) {
-                if constexpr (MULTI)
-                    dsmem_st_async_f4(dsmem_addr(p, 0), v, bar);
-                else
-                    *p = v;
-            };
-            auto put1 = [&](int* p, int v) {
-                if constexpr (MULTI)
-                    dsmem_st_async_i(dsmem_addr(p, 0), v, bar);
-                else
-                    *p = v;
-            };
-            if (MULTI && lane == 0) // share and count; ctl; the recent pairs
-                dsmem_mbar_arrive_expect_tx(bar, 20u + (part == 0 ? 16u + (skip ? 0u : rc > 32 ? 1280u : 640u) : 0u));
-            if (part == 0) {
-                // the recent pairs, with their members outside the lag: their phases are final
-                auto post = [&](int at, uint4 r) {
-                    const int t = r.z & 0x1fff, ku = (r.z >> 13) & 63, kv = (r.z >> 19) & 63;
-                    const float4 sv = vt[t];
-                    float2 x = make_float2(sv.x, sv.y); // v, unless u is the one outside the lag
-                    if (!ku)
-                        x = map_at((long long)m.x - __float_as_int(sv.z));
-                    put4(&ent[s * kRecentMax + at], make_float4(__uint_as_float(r.x), __uint_as_float(r.y), x.x, x.y));
-                    const int own = 2 * (s * kRecentMax + at) + 1, lst = 2 * kRing * kRecentMax;
-                    const unsigned cu = ku ? lst + 2 * ((q - ku) & (kRing - 1)) : own;
-                    const unsigned cv = kv ? lst + 2 * ((q - kv) & (kRing - 1)) : own;
-                    put1(reinterpret_cast<int*>(&ecode[s * kRecentMax + at]),
-                         (int)(cu | cv << 16 | (ku == 1 ? 0x4000u : 0u) | (kv == 1 ? 0x40000000u : 0u)
-                               | ((r.z >> 25) & 1u) << 31));
-                };
-                if (!skip) {
-                    post(lane, ra);
-                    if (rc > 32)
-                        post(lane + 32, rb);
-                }
-                if (lane == 0) {
-                    const int kind = skip ? kSkip : ((m.z >> 16) & 1 && !oor_any ? kFast : kWide);
-                    put4(&ctl[s], make_float4(cur.x, cur.y, __int_as_float(kind),
-                                              __int_as_float(kc | (rc > 32 ? 1 << 8 : 0))));
-                }
-            }
+            skip = __all_sync(0xffffffffu, skip);
             float sr = 0.f, si = 0.f;
             int cnt = 0;
-            if (!skip) {
-                const float2* mb = J.pmap + m.x;
-                // NB: words of the longest batch, the others one less (GUARD:
-                // any number).  OOR: look for out-of-range elements too.
-                auto sum_pairs = [&](auto nbw, auto guard, auto oor) {
-                    constexpr int NB = decltype(nbw)::value;
-                    constexpr bool GUARD = decltype(guard)::value, OOR = decltype(oor)::value;
-                    for (int b = 0; b < nbat; ++b) {
-                        const int i0 = wb + b * (we - wb) / nbat, n = wb + (b + 1) * (we - wb) / nbat - i0;
-                        const float2* pw = prow + 32 * i0;
-                        const float4* vw = vt + 32 * i0 + lane;
-                        float2 bh[NB], u[NB], v[NB];
+            const float2* mb = J.pmap + m.x;
+            const float2* prow = J.plan + (long long)q * nslots + lane;
+            // the part's words in order, NB gathers at a time
+            auto sum_pairs = [&](auto nb, auto rowed) {
+                constexpr int NB = decltype(nb)::value;
+                constexpr bool ROW = decltype(rowed)::value;
+                for (int i0 = wb; i0 < we; i0 += NB) {
+                    float2 u[NB], bh[ROW ? 1 : NB];
 #pragma unroll
-                        for (int k = 0; k < NB; ++k) {
-                            const int i = (GUARD || k == NB - 1) && k >= n ? 0 : 32 * k;
-                            const float4 sl = vw[i];
-                            v[k] = make_float2(sl.x, sl.y);
-                            bh[k] = ld_stream(pw + i);
-                            const float2* up = mb - __float_as_int(sl.z);
-                            u[k] = MULTI ? __ldcg(up) : *up;
-                        }
-#pragma unroll
-                        for (int k = 0; k < NB; ++k) {
-                            const bool in = !((GUARD || k == NB - 1) && k >= n);
-                            const float2 p = pair_product(u[k], v[k], bh[k].x, bh[k].y);
-                            const float n2 = norm2(p);
-                            const float r = rsqrt_ftz(n2);
-                            if (in && !isnan(n2)) {
-                                sr = fmaf(p.x, r, sr);
-                                si = fmaf(p.y, r, si);
-                                ++cnt;
-                            }
-                            if constexpr (OOR)
-                                check_oor(in && __float_as_uint(bh[k].x) == kOorBits, u[k], v[k]);
-                        }
+                    for (int k = 0; k < NB; ++k) {
+                        const int i = i0 + k < we ? 32 * (i0 + k) : 32 * i0;
+                        const float2* up = mb - voff[i + lane];
+                        u[k] = MULTI ? __ldcg(up) : *up;
+                        if constexpr (!ROW)
+                            bh[k] = ld_stream(prow + i);
                     }
-                };
+#pragma unroll
+                    for (int k = 0; k < NB; ++k) { // no branch: the words' latencies overlap
+                        const bool in = i0 + k < we;
+                        const int i = in ? i0 + k : i0;
+                        const float2 v = vt[32 * i + lane];
+                        float2 b;
+                        if constexpr (ROW)
+                            b = row[32 * (i - wb) + lane];
+                        else
+                            b = bh[k];
+                        const float2 p = pair_product(u[k], v, b.x, b.y);
+                        const float n2 = norm2(p);
+                        const float r = rsqrt_ftz(n2);
+                        const bool use = in && !isnan(n2);
+                        sr = use ? fmaf(p.x, r, sr) : sr;
+                        si = use ? fmaf(p.y, r, si) : si;
+                        cnt += use ? 1 : 0;
+                    }
+                }
+            };
+            if (flying) { // also of a visit that is skipped: the buffer must be free for the next
+                if (!__all_sync(0xffffffffu, wait_until([&] { return mbar_try_wait(&row_bar[warp], phase); }, 0u) ? 1 : 0))
+                    break;
+                phase ^= 1u;
+                flying = false;
+            }
+            if (!skip) {
                 using Yes = std::true_type;
                 using No = std::false_type;
-                if (oor_any)
-                    sum_pairs(std::integral_constant<int, kB> {}, Yes {}, Yes {});
-                else if (nbw == 10)
-                    sum_pairs(std::integral_constant<int, 10> {}, No {}, No {});
-                else if (nbw == 9)
-                    sum_pairs(std::integral_constant<int, 9> {}, No {}, No {});
-                else if (nbw == 8)
-                    sum_pairs(std::integral_constant<int, 8> {}, No {}, No {});
-                else if (nbw == 7)
-                    sum_pairs(std::integral_constant<int, 7> {}, No {}, No {});
+                if (!staged)
+                    sum_pairs(std::integral_constant<int, kBDirect> {}, No {});
+                else if (nbw <= 10)
+                    sum_pairs(std::integral_constant<int, 10> {}, Yes {});
+                else if (nbw <= 18)
+                    sum_pairs(std::integral_constant<int, 18> {}, Yes {});
                 else
-                    sum_pairs(std::integral_constant<int, 6> {}, Yes {}, No {});
+                    sum_pairs(std::integral_constant<int, kB> {}, Yes {});
+                if (oor_any) // pairs that get_element would throw for
+                    for (int i = wb; i < we; ++i) {
+                        const float2 v = vt[32 * i + lane], *up = mb - voff[32 * i + lane];
+                        check_oor(__float_as_uint(ld_stream(prow + 32 * i).x) == kOorBits, MULTI ? __ldcg(up) : *up, v);
+                    }
+                if (kc == 0 && !isnan(cur.x)) { // it had its phase
+                    sr = si = 0.f;
+                    cnt = 0;
+                }
+            }
+            __syncwarp();
+            nx = nanf_;
+            if (q + at_once < J.nvisits) {
+                stage(q + at_once, nm);
+                if (nm.x >= 0)
+                    nx = map_at(nm.x).x; // on its way during what follows
             }
             // float-float over the lanes, lane 0's order
             float rh = sr, rl = 0.f, ih = si, il = 0.f;
@@ -923,16 +1055,30 @@ __global__ void __launch_bounds__(kRecoThreads, 1) phase_walk_kernel(const RecoJ
                 ff_add(ih, il, c, f);
             }
             cnt = __reduce_add_sync(0xffffffffu, cnt);
+            const int s = q & (kRing - 1);
             if (lane == 0) {
-                put4(&shr[part][s], make_float4(rh, rl, ih, il));
-                put1(&shn[part][s], cnt);
-            }
-            if constexpr (!MULTI) {
-                __syncwarp();
-                if (lane == 0)
+                const float4 sum = make_float4(rh, rl, ih, il), c = make_float4(__int_as_float(cnt), cur.x, cur.y, 0.f);
+                if constexpr (MULTI) {
+                    const uint32_t bar = dsmem_addr(&ring_bar[s], 0);
+                    dsmem_mbar_arrive_expect_tx(bar, part == 0 ? 32u : 20u);
+                    dsmem_st_async_f4(dsmem_addr(&shr[part][s], 0), sum, bar);
+                    if (part == 0)
+                        dsmem_st_async_f4(dsmem_addr(&shc[s], 0), c, bar);
+                    else
+                        dsmem_st_async_i(dsmem_addr(&shn[part][s], 0), cnt, bar);
+                } else {
+                    shr[part][s] = sum;
+                    if (part == 0)
+                        shc[s] = c;
+                    else
+                        shn[part][s] = cnt;
                     st_release_cta(&tag_s[part][s], q + 1);
+                }
             }
+            __syncwarp();
         }
+        if (flying) // the walk was given up: no copy outlives its CTA
+            mbar_wait_bounded(&row_bar[warp], phase, kRecoWaitNs);
     }
     if constexpr (MULTI)
         cluster_sync_all(); // no CTA touches another's shared memory after this
@@ -1163,10 +1309,10 @@ cudaError_t launch_phase_reco(const RecoJob* jobs_dev, int njobs, int max_W, int
     const int nv = (max_De + 1) * (max_De + 1), nslots = (nv + 31) / 32 * 32;
     spiral_plan_kernel<<<dim3(1216, njobs), 32 * kPlanWarps, sizeof(int) * nslots, st>>>(jobs_dev);
     note_launches(1);
-    const size_t smem = walk_smem(nslots);
-    // the limit is that of the largest depth (the attribute is per function; a
-    // launch of another shape must never lower it under this one)
-    const int smem_max = (int)walk_smem(kMaxWords * 32);
+    // the limit is that of any depth (the attribute is per function; a launch of
+    // another shape must never lower it under this one)
+    const int smem_max = (int)(box_bytes(kMaxWords * 32) + (size_t)kRowWords * 256 * (kRecoThreads / 32));
+    size_t smem = walk_smem(max_De, nslots, true);
     int ncta = walk_ctas(max_De);
     cudaError_t e = cudaSuccess;
     if (ncta > 1) {
@@ -1202,6 +1348,7 @@ cudaError_t launch_phase_reco(const RecoJob* jobs_dev, int njobs, int max_W, int
         e = cudaFuncSetAttribute(phase_walk_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
         if (e != cudaSuccess)
             return e;
+        smem = walk_smem(max_De, nslots, false);
         phase_walk_kernel<false><<<njobs, kRecoThreads, smem, st>>>(jobs_dev);
         note_launches(1);
     }

@@ -56,3 +56,17 @@ def test_walk_shapes(smip, oracle, W, H, D, R, holes):
     assert e.max() <= 1e-3 and np.sqrt((e ** 2).mean()) <= 1e-4, (e.max(), np.sqrt((e ** 2).mean()))
     assert np.all(got[~m] == 0) and np.all(gcs[~m] == 0)
     assert np.abs(gcs[m] - cs[m]).max() <= 1e-3
+
+
+# a summing warp's plan row: one batch (20 words), two, the longest row that is
+# kept in shared memory (39 words) and the first that is not (43)
+@pytest.mark.parametrize("W,H,D,R", [(80, 64, 24, 32), (64, 80, 32, 32), (80, 81, 34, 36), (81, 80, 36, 36)])
+def test_walk_rows(smip, oracle, W, H, D, R):
+    B = bispectrum(oracle, W, H, D, 5 * W + H + D)
+    ph, fl, cs = oracle.reconstruct_phases(B, W, H, D, R)
+    got, gfl, gcs = smip.reconstruct_phases(B, W, H, D, R)
+    assert np.array_equal(gfl, fl)
+    m = fl > 0
+    e = phase_err(got, ph, m)
+    assert e.max() <= 1e-3 and np.sqrt((e ** 2).mean()) <= 1e-4, (e.max(), np.sqrt((e ** 2).mean()))
+    assert np.abs(gcs[m] - cs[m]).max() <= 1e-3
