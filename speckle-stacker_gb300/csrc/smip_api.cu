@@ -1056,9 +1056,11 @@ extern "C" int smip_stack_reset(smip_stack_t s)
     CUDA_TRY(cudaStreamSynchronize(s->st));
     if (s->cst) // frames copied for a batch that the reset drops
         CUDA_TRY(cudaStreamSynchronize(s->cst));
+    if (s->rst) // a phase recovery that no call has waited for reads B and C and may record an error
+        CUDA_TRY(cudaStreamSynchronize(s->rst));
     if ((rc = s->collect_timing()))
         return rc;
-    *s->err = 0; // the stream is idle
+    *s->err = 0; // all of the stack's streams are idle
     // (the tile counters too: a launch that stopped early may leave parts counted)
     CUDA_TRY(cudaMemsetAsync(s->zeroed, 0, s->zeroed_bytes, s->st));
     s->nframes = 0;
@@ -1428,17 +1430,22 @@ extern "C" int smip_stack_bispectrum(smip_stack_t s, float* out)
 }
 
 // Phase recovery (and the final image) run on the stack's high-priority
-// stream: the walk is one CTA per job, and when several jobs share the GPU
-// its blocks are scheduled ahead of pending accumulation blocks of other
-// jobs.  The stack's stream is idle here (synchronised); rejoin_stream
-// orders the later downloads on it after this work.
-static int stack_reco(smip_stack_t s, double R)
+// stream: the walk is a cluster of two, four or eight CTAs per job, and when
+// several jobs share the GPU its blocks are scheduled ahead of pending
+// accumulation blocks of other jobs.  The stack's stream is idle here
+// (synchronised); rejoin_stream orders the later downloads on it after this
+// work.  A call that is refused launches nothing.
+static int stack_reco(smip_stack_t s, double R, bool image)
 {
     int rc = smip_stack_sync(s);
     if (rc || (rc = need_frames(s)))
         return rc;
     if (!(R >= 0.0))
         return fail(SMIP_E_INVALID_ARGUMENT, "reco_radius must be >= 0");
+    if (image && s->mode != 1)
+        return fail(SMIP_E_BAD_CALL, "the final image needs the power spectrum of pushed frames");
+    if (image && !(R > 0.0))
+        return fail(SMIP_E_DOMAIN, "WindowFunction aperture size <= 0");
     if ((rc = prepare_reco(s, R)) || (rc = normalize_bispec(s, s->rst)))
         return rc;
     return s->reco.run(s->Bn, R, s->err, s->rst);
@@ -1453,7 +1460,7 @@ static int rejoin_stream(smip_stack_t s)
 
 extern "C" int smip_stack_reconstruct(smip_stack_t s, double R, double* phases, unsigned char* flags, double* cons)
 {
-    int rc = stack_reco(s, R);
+    int rc = stack_reco(s, R, false);
     if (rc || (rc = rejoin_stream(s)))
         return rc;
     if ((rc = s->reco.download(phases, flags, cons, s->st)))
@@ -1464,13 +1471,9 @@ extern "C" int smip_stack_reconstruct(smip_stack_t s, double R, double* phases, 
 extern "C" int smip_stack_finish(smip_stack_t s, double R, double* image, double* phases, unsigned char* flags,
                                  double* cons)
 {
-    int rc = stack_reco(s, R);
+    int rc = stack_reco(s, R, true);
     if (rc)
         return rc;
-    if (s->mode != 1)
-        return fail(SMIP_E_BAD_CALL, "the final image needs the power spectrum of pushed frames");
-    if (!(R > 0.0))
-        return fail(SMIP_E_DOMAIN, "WindowFunction aperture size <= 0");
     const size_t n = s->frame_elems();
     const double pnorm = (double)((size_t)s->nframes * n);
     CUDA_TRY(launch_finish(s->P, pnorm, s->reco.phases, 2.0 * R, s->g, s->Z, nullptr, s->maxbuf, s->ctx->tw64, s->rst,
