@@ -160,7 +160,7 @@ constexpr unsigned kUnusable = 0x7fc00000u;
 constexpr unsigned kOorBits = 0x7fc00001u;
 constexpr int kPlanWarps = 8;
 
-// rec code: slot t (13 bits) | ku << 13 | kv << 19 | phasor is kOorBits << 25
+// rec code: slot t (13 bits) | ku << 13 | kv << 19
 // meta.z: recent pairs | kc << 8 | fast << 16 | runnable << 17
 __global__ void __launch_bounds__(32 * kPlanWarps) spiral_plan_kernel(const RecoJob* __restrict__ jobs)
 {
@@ -312,8 +312,7 @@ __global__ void __launch_bounds__(32 * kPlanWarps) spiral_plan_kernel(const Reco
             const unsigned bits = mask[i];
             if ((bits >> lane) & 1u) {
                 const int pos = before + __popc(bits & ((1u << lane) - 1u));
-                const unsigned c = code[pos] | (__float_as_uint(out.x) == kOorBits ? 1u << 25 : 0u);
-                rec[pos ^ perm] = make_uint4(__float_as_uint(out.x), __float_as_uint(out.y), c, 0u);
+                rec[pos ^ perm] = make_uint4(__float_as_uint(out.x), __float_as_uint(out.y), code[pos], 0u);
                 out = nan2;
             }
             before += __popc(bits);
@@ -967,7 +966,10 @@ __global__ void __launch_bounds__(kRecoThreads, 1) phase_walk_kernel(const RecoJ
                                 return pr >= q - kRecoLag;
                             }, 20u) ? 1 : 0))
                 break;
-            if (oor_any && !skip && kc == 0) // the errors of a point that has its phase do not count
+            // The errors of a point that has its phase do not count, however long
+            // ago it was visited.  One that gets its phase within the lag was
+            // formed then from every pair that is summed here, errors included.
+            if (oor_any && !skip)
                 skip = !isnan(map_at(m.x).x);
             float2 cur = make_float2(nanf_, nanf_); // waited for at the end
             if (m.x >= 0)
