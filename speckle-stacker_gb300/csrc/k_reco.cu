@@ -152,12 +152,15 @@ __global__ void __launch_bounds__(256) reco_plan_kernel(const RecoJob* __restric
 // A visit with at most 32 recent pairs of which at most one has age 1 is
 // "fast": its list is stored permuted by XOR with that pair's position, which
 // puts the pair into lane 0 and leaves the order of a butterfly sum as it is.
-// A phasor that is NaN (Bispectrum::get_element would throw, or B is not a
-// number) has the payload kOorBits and raises J.oor.
+// A phasor whose real part is NaN (Bispectrum::get_element would throw, or B is
+// not a number) has the payload kOorBits; one whose imaginary part alone is NaN
+// (that of B is infinite) has kNanBits: its pair counts and makes the point's sum
+// NaN.  Both raise J.oor, which has the walk look for them.
 // Bound by the scattered reads of B (one 32-byte sector per pair): 64 M pairs
 // at 256 x 256, d = 32.
 constexpr unsigned kUnusable = 0x7fc00000u;
 constexpr unsigned kOorBits = 0x7fc00001u;
+constexpr unsigned kNanBits = 0x7fc00002u;
 constexpr int kPlanWarps = 8;
 
 // rec code: slot t (13 bits) | ku << 13 | kv << 19
@@ -292,19 +295,19 @@ __global__ void __launch_bounds__(32 * kPlanWarps) spiral_plan_kernel(const Reco
                 if (in_map(ux, uy)) {
                     int cj = 0;
                     const long long off = bispec_get_offset(d, ux, uy, vx, vy, &cj);
-                    bool bad = off < 0;
+                    unsigned bad = off < 0 ? kOorBits : 0u;
                     if (!bad) {
                         float2 b = __ldg(&J.B[off]);
                         if (cj)
                             b.y = -b.y;
                         float2 bh;
                         if (unit_phasor(b, &bh)) {
-                            bad = isnan(bh.x);
+                            bad = isnan(bh.x) ? kOorBits : isnan(bh.y) ? kNanBits : 0u;
                             out = bh;
                         }
                     }
                     if (bad) {
-                        out = make_float2(__uint_as_float(kOorBits), __uint_as_float(kOorBits));
+                        out = make_float2(__uint_as_float(bad), __uint_as_float(bad));
                         oor = true;
                     }
                 }
@@ -570,10 +573,14 @@ __global__ void __launch_bounds__(kRecoThreads, 1) phase_walk_kernel(const RecoJ
             }
         }
     };
-    const bool oor_any = *J.oor != 0;
-    auto check_oor = [&](bool is_oor, float2 U, float2 V) { // get_element would throw in a pair that is used
-        if (is_oor && !isnan(U.x) && !isnan(V.x))
+    const bool oor_any = *J.oor != 0; // some phasor is marked
+    // a pair of a marked phasor b, used: true where it makes the sum NaN
+    auto marked = [&](float bx, float2 U, float2 V) {
+        const unsigned b = __float_as_uint(bx);
+        const bool used = (b == kOorBits || b == kNanBits) && !isnan(U.x) && !isnan(V.x);
+        if (used && b == kOorBits) // get_element would throw
             record_error(J.err, SMIP_DEV_ERR_OUT_OF_RANGE);
+        return used && b == kNanBits;
     };
 
     // which warp does what (a nibble each): 0 the serial warp, 1 the writer,
@@ -720,8 +727,12 @@ __global__ void __launch_bounds__(kRecoThreads, 1) phase_walk_kernel(const RecoJ
             const float4 own = res_p[(q - kc) & (kRing - 1)];
             float2 pa, pb, kept;
             float ra, rb;
-            const bool oka = term(Ua, Va, make_float2(ba.x, ba.y), pa, ra);
-            const bool okb = term(Ub, Vb, make_float2(bb.x, bb.y), pb, rb) && two;
+            bool oka = term(Ua, Va, make_float2(ba.x, ba.y), pa, ra);
+            bool okb = term(Ub, Vb, make_float2(bb.x, bb.y), pb, rb) && two;
+            if (oor_any && q < J.nvisits && !(kc && !isnan(own.x))) { // (a NaN term is then a pair like any other)
+                oka = marked(ba.x, Ua, Va) || oka;
+                okb = (two && marked(bb.x, Ub, Vb)) || okb;
+            }
             float sr = oka ? fmaf(pa.x, ra, 0.f) : 0.f, si = oka ? fmaf(pa.y, ra, 0.f) : 0.f;
             sr = okb ? fmaf(pb.x, rb, sr) : sr;
             si = okb ? fmaf(pb.y, rb, si) : si;
@@ -735,9 +746,6 @@ __global__ void __launch_bounds__(kRecoThreads, 1) phase_walk_kernel(const RecoJ
             if (kc && !isnan(own.x)) { // its point, visited within the lag, has its phase
                 now = make_float2(own.x, own.y);
                 cnt = 0.f;
-            } else if (oor_any && q < J.nvisits) {
-                check_oor(__float_as_uint(ba.x) == kOorBits, Ua, Va);
-                check_oor(two && __float_as_uint(bb.x) == kOorBits, Ub, Vb);
             }
             const float4* ne = &ent[s1 * kRecentMax + lane];
             early(phase_at(lc.x), phase_at(lc.y), make_float2(ne->x, ne->y));
@@ -1030,10 +1038,13 @@ __global__ void __launch_bounds__(kRecoThreads, 1) phase_walk_kernel(const RecoJ
                     sum_pairs(std::integral_constant<int, 18> {}, Yes {});
                 else
                     sum_pairs(std::integral_constant<int, kB> {}, Yes {});
-                if (oor_any) // pairs that get_element would throw for
+                if (oor_any)
                     for (int i = wb; i < we; ++i) {
                         const float2 v = vt[32 * i + lane], *up = mb - voff[32 * i + lane];
-                        check_oor(__float_as_uint(ld_stream(prow + 32 * i).x) == kOorBits, MULTI ? __ldcg(up) : *up, v);
+                        if (marked(ld_stream(prow + 32 * i).x, MULTI ? __ldcg(up) : *up, v)) {
+                            sr = si = nanf_;
+                            ++cnt;
+                        }
                     }
                 if (kc == 0 && !isnan(cur.x)) { // it had its phase
                     sr = si = 0.f;

@@ -183,7 +183,7 @@ struct RecoJob {
     // the spiral walk's visits (k_reco.cu, spiral_plan_kernel)
     uint4* rec;          // [nvisits][kRecentMax] recent pairs
     int4* meta;          // [nvisits]
-    int* oor;            // some pair's bispectrum element is out of range
+    int* oor;            // some pair's bispectrum element is out of range or not finite
 };
 constexpr int kRecoLag = 32;     // visits between a point's phase and the parallel stage's use of it
 constexpr int kRecentMax = 64;   // recent pairs per visit: at most 32 by u and 32 by v

@@ -2,7 +2,10 @@
 
 An element with an infinite real part is reported like one outside the array,
 but only if a point is formed from it (calc_phase leaves a point that has its
-phase alone, phasereco.h:81-84).
+phase alone, phasereco.h:81-84).  One with an infinite imaginary part and a
+finite real part has the phasor (0, NaN): a point that is formed from it has a
+consistency that is NaN and the phase zero, and so have the points formed from
+that one.
 """
 import numpy as np
 import pytest
@@ -44,3 +47,21 @@ def test_errors_that_count(smip):
     B[smip.bispec_offsets(16, 16, 8, [[1, 0, 1, 0]])[0]] = complex(np.inf, 0)  # forms (2, 0), the spiral's first point
     with pytest.raises(smip.OutOfRange):
         smip.reconstruct_phases(B, 16, 16, 8, 6)
+
+
+# recent pairs and older ones; a point near the origin and points of the last
+# turns; a summing warp's plan row in one part and in several
+@pytest.mark.parametrize("W,H,D,R,pair", [
+    (32, 32, 8, 12, (9, 2, 2, -1)), (32, 32, 8, 12, (11, -3, -1, 4)), (32, 32, 8, 12, (2, 0, 1, 1)),
+    (48, 40, 14, 18, (-17, 2, 1, 1)), (64, 64, 24, 20, (14, 5, 4, 3)), (96, 96, 40, 24, (10, -10, 10, 3))])
+def test_infinite_imaginary_part(smip, oracle, W, H, D, R, pair):
+    B = sparse(W, H, D, 0.0, W + D)
+    off = smip.bispec_offsets(W, H, D, [pair])[0][0]
+    B[off] = complex(0.5, np.inf)
+    ph, fl, cs = oracle.reconstruct_phases(B, W, H, D, R)
+    lost = np.isnan(cs)
+    assert lost.any()
+    got, gfl, gcs = smip.reconstruct_phases(B, W, H, D, R)
+    assert np.array_equal(gfl, fl)
+    assert np.array_equal(np.isnan(gcs), lost)
+    assert np.array_equal(got[lost], ph[lost]) and np.all(got[lost] == 0)
