@@ -58,10 +58,12 @@ cudaError_t launch_bounded_wait_probe(int* err, const int* never, double timeout
 }
 
 // ------------------------------------------------------- normalise, merge
-// (B - C) / n, rounded once: the difference is formed exactly as a float pair
-// and multiplied by 1/n as one, on the FP32 pipes (GB300's FP64 rate bound this
-// kernel: 351 us at 256 x 256, d = 32, 1.3 TB/s; now HBM does).  Values near the
-// ends of the FP32 range, infinities and NaN take the FP64 form.
+// (B - C) / n as FP64 arithmetic and one rounding give it, to the bit, but on the
+// FP32 pipes (GB300's FP64 rate bound this kernel: 351 us at 256 x 256, d = 32,
+// 1.3 TB/s; now HBM does).  The difference is an exact float pair, its product
+// with 1/n as a float pair is within 2^-45 of FP64's.  Where that leaves the
+// rounding open (a value that close to the middle of two floats), and for values
+// so small that the pair loses bits, infinities and NaN, the FP64 form decides.
 // (a call, so that the compiler does not compute it beside the other form)
 __device__ __noinline__ float normalized_f64(float b, float c, double inv_n)
 {
@@ -72,11 +74,11 @@ __device__ __forceinline__ float normalized(float b, float c, float ih, float il
     float s, e;
     two_sum(b, -c, s, e);
     const float p = __fmul_rn(s, ih);
-    const float r = __fadd_rn(p, fmaf(e, ih, fmaf(s, il, fmaf(s, ih, -p))));
-    const float m = fabsf(s);
-    if (m <= 1e37f && (m >= 1e-24f || m == 0.f))
+    const float q = fmaf(e, ih, fmaf(s, il, fmaf(s, ih, -p))), t = __fmul_rn(fabsf(p), 0x1p-44f);
+    const float r = __fadd_rn(p, __fadd_rn(q, -t));
+    if (r == __fadd_rn(p, __fadd_rn(q, t)) && fabsf(p) >= 0x1p-80f)
         return r;
-    return normalized_f64(b, c, inv_n);
+    return s == 0.f ? p : normalized_f64(b, c, inv_n);
 }
 
 __global__ void __launch_bounds__(256) bispec_normalize_kernel(const float2* __restrict__ B, const float2* __restrict__ C,
