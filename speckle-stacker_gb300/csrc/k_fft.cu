@@ -53,10 +53,11 @@ __device__ __forceinline__ float2 df_round(const dfc& v) { return make_float2(v.
 template <typename T>
 __global__ void __launch_bounds__(256, 4) row_pass_kernel(const T* __restrict__ frames, long long fstride, int logW, int H,
                                                         int hw, dfc* __restrict__ Gt, const dfc* __restrict__ tw_g,
-                                                        T* __restrict__ copy_out, float* __restrict__ rowsq)
+                                                        T* __restrict__ copy_out, SqSum<T>* __restrict__ rowsq)
 {
     extern __shared__ dfc smdf[];
-    float sq = 0.f; // of this thread's pixels, for the correlation's error bound (k_xcorr.cu)
+    __shared__ SqSum<T> sqpart[8];
+    SqSum<T> sq {}; // of this thread's pixels, for the correlation's error bound (k_xcorr.cu)
     const int W = 1 << logW;
     dfc* tw = smdf;                                // W - 1, stage-packed (+1 spare)
     dfc* lines = smdf + W;                         // [kRowBlock/2][pad8(W) + 1]
@@ -101,21 +102,22 @@ __global__ void __launch_bounds__(256, 4) row_pass_kernel(const T* __restrict__ 
                 dfc d;
                 d.h = make_float2((float)p0[e], (float)p1[e]);
                 d.l = make_float2(0.f, 0.f);
-                sq = fmaf(d.h.x, d.h.x, fmaf(d.h.y, d.h.y, sq));
+                sq_add(sq, p0[e]);
+                sq_add(sq, p1[e]);
                 L[pad8(bitrev(x0 + e, logW))] = d;
             }
         }
     } else {
         for (int idx = threadIdx.x; idx < kRowBlock * W; idx += blockDim.x) {
-            const float2 v = pix_df(fr, idx);
-            sq = fmaf(v.x, v.x, sq);
-            put(idx, v);
+            sq_add(sq, fr[idx]);
+            put(idx, pix_df(fr, idx));
             if (co)
                 co[idx] = fr[idx];
         }
     }
-    store_block_sum(sq, rowsq + (long long)f * gridDim.x + blockIdx.x);
+    sq_store_warp(sq, sqpart);
     __syncthreads();
+    sq_store_block(sqpart, rowsq + (long long)f * gridDim.x + blockIdx.x);
     fft_passes(lines, logW, kRowBlock / 2, LW, tw, kTwLog, -1);
     dfc* out = Gt + (long long)f * hw * H;
     for (int idx = threadIdx.x; idx < hw * kRowBlock; idx += blockDim.x) {
@@ -363,7 +365,7 @@ static size_t xcorr_rows_smem(int W) { return sizeof(float2) * (W + (W / 2 + 1) 
 int row_blocks(const Geometry& g) { return g.generic ? gen_row_blocks(g) : g.H / kRowBlock; }
 
 cudaError_t launch_row_pass(int dtype, const void* frames, long long fstride, int nframes, const Geometry& g, dfc* Gt,
-                            float* rowsq, const dfc* twdf, cudaStream_t st, void* copy_out)
+                            void* rowsq, const dfc* twdf, cudaStream_t st, void* copy_out)
 {
     const dim3 grid(g.H / kRowBlock, nframes);
     const size_t smem = row_pass_smem(g.W), smem_max = row_pass_smem(1 << kMaxLog);
@@ -372,22 +374,22 @@ cudaError_t launch_row_pass(int dtype, const void* frames, long long fstride, in
     case 0:
         if ((e = allow_smem(row_pass_kernel<uint8_t>, smem_max)) != cudaSuccess) return e;
         row_pass_kernel<uint8_t><<<grid, 256, smem, st>>>((const uint8_t*)frames, fstride, g.logW, g.H, g.hw, Gt, twdf,
-                                                          (uint8_t*)copy_out, rowsq);
+                                                          (uint8_t*)copy_out, (SqSum<uint8_t>*)rowsq);
         break;
     case 1:
         if ((e = allow_smem(row_pass_kernel<uint16_t>, smem_max)) != cudaSuccess) return e;
         row_pass_kernel<uint16_t><<<grid, 256, smem, st>>>((const uint16_t*)frames, fstride, g.logW, g.H, g.hw, Gt, twdf,
-                                                           (uint16_t*)copy_out, rowsq);
+                                                           (uint16_t*)copy_out, (SqSum<uint16_t>*)rowsq);
         break;
     case 2:
         if ((e = allow_smem(row_pass_kernel<float>, smem_max)) != cudaSuccess) return e;
         row_pass_kernel<float><<<grid, 256, smem, st>>>((const float*)frames, fstride, g.logW, g.H, g.hw, Gt, twdf,
-                                                        (float*)copy_out, rowsq);
+                                                        (float*)copy_out, (SqSum<float>*)rowsq);
         break;
     default:
         if ((e = allow_smem(row_pass_kernel<double>, smem_max)) != cudaSuccess) return e;
         row_pass_kernel<double><<<grid, 256, smem, st>>>((const double*)frames, fstride, g.logW, g.H, g.hw, Gt, twdf,
-                                                         (double*)copy_out, rowsq);
+                                                         (double*)copy_out, (SqSum<double>*)rowsq);
         break;
     }
     note_launches(1);

@@ -285,10 +285,11 @@ template <typename T>
 __global__ void __launch_bounds__(256, 4) gen_row_kernel(const T* __restrict__ frames, long long fstride, int H, int hw,
                                                       int rb, const GenPlan pw, const dfc* __restrict__ tw_g,
                                                       dfc* __restrict__ Gt, T* __restrict__ copy_out,
-                                                      float* __restrict__ rowsq)
+                                                      SqSum<T>* __restrict__ rowsq)
 {
     extern __shared__ dfc smg[];
-    float sq = 0.f; // of this thread's pixels, for the correlation's error bound (k_xcorr.cu)
+    __shared__ SqSum<T> sqpart[8];
+    SqSum<T> sq {}; // of this thread's pixels, for the correlation's error bound (k_xcorr.cu)
     const int W = pw.L;
     dfc* tw = smg;
     dfc* X = tw + W;
@@ -302,19 +303,21 @@ __global__ void __launch_bounds__(256, 4) gen_row_kernel(const T* __restrict__ f
     for (int i = threadIdx.x; i < nl * W; i += blockDim.x) {
         const int l = i / W, x = i - l * W, at = 2 * l * W + x;
         const bool two = 2 * l + 1 < nr; // the last row of an odd block goes alone
-        const float2 p0 = pix_pair(fr, at), p1 = two ? pix_pair(fr, at + W) : make_float2(0.f, 0.f);
+        const T v0 = fr[at], v1 = two ? fr[at + W] : T(0);
+        const float2 p0 = pix_pair(&v0, 0), p1 = pix_pair(&v1, 0);
         dfc d;
         d.h = make_float2(p0.x, p1.x);
         d.l = make_float2(p0.y, p1.y);
-        sq = fmaf(p0.x, p0.x, fmaf(p1.x, p1.x, sq));
+        sq_add(sq, v0);
+        sq_add(sq, v1);
         X[i] = d;
         if (co) {
-            co[at] = fr[at];
+            co[at] = v0;
             if (two)
-                co[at + W] = fr[at + W];
+                co[at + W] = v1;
         }
     }
-    store_block_sum(sq, rowsq + (long long)f * gridDim.x + blockIdx.x);
+    sq_store_warp(sq, sqpart);
     __syncthreads();
     const dfc* Z = stockham(X, Y, pw, nl, W, tw, -1);
     dfc* out = Gt + (long long)f * hw * H;
@@ -333,6 +336,8 @@ __global__ void __launch_bounds__(256, 4) gen_row_kernel(const T* __restrict__ f
         g.h.x *= 0.5f; g.l.x *= 0.5f; g.h.y *= 0.5f; g.l.y *= 0.5f;
         out[(long long)a * H + y0 + r] = g;
     }
+    // (here: before the transform it costs spills, 110 us at 200 frames of 640 x 480)
+    sq_store_block(sqpart, rowsq + (long long)f * gridDim.x + blockIdx.x);
 }
 
 // ------------------------------------------------------------- column pass
@@ -560,7 +565,7 @@ size_t gen_max_smem() { return kGenSmem; }
 int gen_row_blocks(const Geometry& g) { return (g.H + row_block(g.W) - 1) / row_block(g.W); }
 
 cudaError_t launch_gen_row_pass(int dtype, const void* frames, long long fstride, int nframes, const Geometry& g,
-                                dfc* Gt, float* rowsq, const dfc* twW, cudaStream_t st, void* copy_out)
+                                dfc* Gt, void* rowsq, const dfc* twW, cudaStream_t st, void* copy_out)
 {
     const int rb = row_block(g.W);
     const dim3 grid((g.H + rb - 1) / rb, nframes);
@@ -570,7 +575,7 @@ cudaError_t launch_gen_row_pass(int dtype, const void* frames, long long fstride
     if ((e = allow(gen_row_kernel<TY>, kGenSmem)) != cudaSuccess)                                                 \
         return e;                                                                                                  \
     gen_row_kernel<TY><<<grid, 256, smem, st>>>((const TY*)frames, fstride, g.H, g.hw, rb, g.pW, twW, Gt,         \
-                                                (TY*)copy_out, rowsq);
+                                                (TY*)copy_out, (SqSum<TY>*)rowsq);
     switch (dtype) {
     case 0: SMIP_GEN_ROW(uint8_t) break;
     case 1: SMIP_GEN_ROW(uint16_t) break;

@@ -155,21 +155,20 @@ template <typename T> __device__ double frame_sumsq(const T* __restrict__ p, int
     return block_sum(s, red);
 }
 
-// A frame's sum of squares from the row pass's sums of its row blocks: FP32,
-// within 1e-3 of the exact one, which the bound below allows for.  Every warp
-// forms it for itself (the same additions, so the same bits).
-__device__ float frame_norm(const float* __restrict__ part, int nsq)
+// A frame's sum of squares from the row pass's sums of its row blocks, by one warp.
+template <typename A> __device__ __forceinline__ A frame_norm(const A* __restrict__ part, int nsq)
 {
-    float s = 0.f;
+    A s {};
     for (int i = threadIdx.x & 31; i < nsq; i += 32)
-        s += part[i];
+        sq_sum(s, part[i]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
-        s += __shfl_xor_sync(0xffffffffu, s, o);
+        sq_fold(s, o);
     return s;
 }
-// sums at the ends of the FP32 range are formed again in FP64
-__device__ __forceinline__ bool norm_ok(float s) { return s > 1e-25f && s < 1e30f; }
+// Sums of floating frames at the ends of the FP32 range are formed again in FP64;
+// those of integer frames are exact.
+template <typename T> __device__ __forceinline__ bool norm_ok(float s) { return sizeof(T) <= 2 || (s > 1e-25f && s < 1e30f); }
 
 // Bound by latency: a frame's pixels are read only where more than one position
 // lies within the bound of the peak (few frames), and the norms come from the row
@@ -184,21 +183,22 @@ __global__ void __launch_bounds__(kShiftThreads) xcorr_shift_kernel(const float*
                                                                      const float* __restrict__ rowmax,
                                                                      const T* __restrict__ frames, long long fstride,
                                                                      const T* __restrict__ ref,
-                                                                     const float* __restrict__ rowsq, int nsq,
-                                                                     const float* __restrict__ refsq, double* ref_sq,
+                                                                     const SqSum<T>* __restrict__ rowsq, int nsq,
+                                                                     const SqSum<T>* __restrict__ refsq, double* ref_sq,
                                                                      int first, int W, int logW, int H,
                                                                      double err_stages, int* __restrict__ shifts)
 {
     using A = typename ExactAcc<T>::type;
     __shared__ A redM[kMulti * 32];
     __shared__ double redD[32];
+    __shared__ float norms[2];
     __shared__ int cand[kMaxCand];
     __shared__ int ncand;
     const int f = blockIdx.x;
     const int n = W * H;
     if (first && f == 0) {
-        const float s32 = frame_norm(refsq, nsq);
-        const double s = norm_ok(s32) ? (double)s32 : frame_sumsq(ref, n, redD);
+        const SqSum<T> part = frame_norm(refsq, nsq);
+        const double s = norm_ok<T>(sq_up(part)) ? sq_value(part) : frame_sumsq(ref, n, redD);
         if (threadIdx.x == 0) {
             *ref_sq = s;
             shifts[0] = 0;
@@ -209,22 +209,34 @@ __global__ void __launch_bounds__(kShiftThreads) xcorr_shift_kernel(const float*
     const float* c = corr + (long long)f * n;
     const float* rm = rowmax + (long long)f * H;
     const T* fr = frames + (long long)f * fstride;
-    // the norms and the FP32 peak from the rows' maxima, by every warp
+    // the FP32 peak from the rows' maxima, by every warp; the norms, rounded up, by
+    // one each
+    if (threadIdx.x < 64) {
+        float s;
+        if (threadIdx.x < 32)
+            s = sq_up(frame_norm(rowsq + (long long)f * nsq, nsq));
+        else
+            s = refsq ? sq_up(frame_norm(refsq, nsq)) : __double2float_ru(*ref_sq);
+        if ((threadIdx.x & 31) == 0)
+            norms[threadIdx.x >> 5] = s;
+    }
     float mx = -INFINITY;
     for (int y = threadIdx.x & 31; y < H; y += 32)
         mx = fmaxf(mx, rm[y]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    const float sq = frame_norm(rowsq + (long long)f * nsq, nsq);
-    const float rsq = refsq ? frame_norm(refsq, nsq) : (float)*ref_sq;
+    __syncthreads();
+    const float sq = norms[0], rsq = norms[1];
     float thr;
-    if (norm_ok(sq) && norm_ok(rsq)) { // FP32, rounded down
-        thr = __fsub_rd(mx, 1.003f * 8.0f * 5.9604644775390625e-08f * (float)err_stages * sqrtf(rsq) * sqrtf(sq) * (float)n);
+    if (norm_ok<T>(sq) && norm_ok<T>(rsq)) {
+        // never above the bound in FP64: the factor covers the roundings here (2^-24
+        // each) and those of a float pair's sum
+        thr = __fsub_rd(mx, 1.000002f * 8.0f * 5.9604644775390625e-08f * (float)err_stages * sqrtf(rsq) * sqrtf(sq) * (float)n);
     } else {
-        const double sqd = norm_ok(sq) ? (double)sq : frame_sumsq(fr, n, redD);
-        const double rsqd = norm_ok(rsq) ? (double)rsq : refsq ? frame_sumsq(ref, n, redD) : *ref_sq;
-        const double tau = 1.002 * 8.0 * 5.9604644775390625e-08 * err_stages * sqrt(rsqd * sqd) * (double)n;
+        const double sqd = norm_ok<T>(sq) ? (double)sq : frame_sumsq(fr, n, redD);
+        const double rsqd = norm_ok<T>(rsq) ? (double)rsq : refsq ? frame_sumsq(ref, n, redD) : *ref_sq;
+        const double tau = 1.000002 * 8.0 * 5.9604644775390625e-08 * err_stages * sqrt(rsqd * sqd) * (double)n;
         thr = (float)((double)mx - tau);
     }
 
@@ -379,7 +391,7 @@ __global__ void __launch_bounds__(256) saa_add_kernel(A* __restrict__ sum, const
 }
 
 cudaError_t launch_xcorr_shift(int dtype, const float* corr, const float* rowmax, const void* frames, long long fstride,
-                               const void* ref, const float* rowsq, int nsq, const float* refsq, double* ref_sq,
+                               const void* ref, const void* rowsq, int nsq, const void* refsq, double* ref_sq,
                                int nframes, int first, const Geometry& g, int* shifts, cudaStream_t st)
 {
     // the correlation's FP32 error grows with the transforms' stages: log2(W H)
@@ -395,10 +407,10 @@ cudaError_t launch_xcorr_shift(int dtype, const float* corr, const float* rowmax
         for (int k = 0; k < g.pH.nf; ++k) stages += of(g.pH.fac[k]);
     }
     switch (dtype) {
-    case 0: xcorr_shift_kernel<uint8_t><<<nframes, kShiftThreads, 0, st>>>(corr, rowmax, (const uint8_t*)frames, fstride, (const uint8_t*)ref, rowsq, nsq, refsq, ref_sq, first, g.W, logW, g.H, stages, shifts); note_launches(1); break;
-    case 1: xcorr_shift_kernel<uint16_t><<<nframes, kShiftThreads, 0, st>>>(corr, rowmax, (const uint16_t*)frames, fstride, (const uint16_t*)ref, rowsq, nsq, refsq, ref_sq, first, g.W, logW, g.H, stages, shifts); note_launches(1); break;
-    case 2: xcorr_shift_kernel<float><<<nframes, kShiftThreads, 0, st>>>(corr, rowmax, (const float*)frames, fstride, (const float*)ref, rowsq, nsq, refsq, ref_sq, first, g.W, logW, g.H, stages, shifts); note_launches(1); break;
-    default: xcorr_shift_kernel<double><<<nframes, kShiftThreads, 0, st>>>(corr, rowmax, (const double*)frames, fstride, (const double*)ref, rowsq, nsq, refsq, ref_sq, first, g.W, logW, g.H, stages, shifts); note_launches(1); break;
+    case 0: xcorr_shift_kernel<uint8_t><<<nframes, kShiftThreads, 0, st>>>(corr, rowmax, (const uint8_t*)frames, fstride, (const uint8_t*)ref, (const SqSum<uint8_t>*)rowsq, nsq, (const SqSum<uint8_t>*)refsq, ref_sq, first, g.W, logW, g.H, stages, shifts); note_launches(1); break;
+    case 1: xcorr_shift_kernel<uint16_t><<<nframes, kShiftThreads, 0, st>>>(corr, rowmax, (const uint16_t*)frames, fstride, (const uint16_t*)ref, (const SqSum<uint16_t>*)rowsq, nsq, (const SqSum<uint16_t>*)refsq, ref_sq, first, g.W, logW, g.H, stages, shifts); note_launches(1); break;
+    case 2: xcorr_shift_kernel<float><<<nframes, kShiftThreads, 0, st>>>(corr, rowmax, (const float*)frames, fstride, (const float*)ref, (const SqSum<float>*)rowsq, nsq, (const SqSum<float>*)refsq, ref_sq, first, g.W, logW, g.H, stages, shifts); note_launches(1); break;
+    default: xcorr_shift_kernel<double><<<nframes, kShiftThreads, 0, st>>>(corr, rowmax, (const double*)frames, fstride, (const double*)ref, (const SqSum<double>*)rowsq, nsq, (const SqSum<double>*)refsq, ref_sq, first, g.W, logW, g.H, stages, shifts); note_launches(1); break;
     }
     return cudaGetLastError();
 }

@@ -541,7 +541,7 @@ struct smip_stack {
     float2 *T = nullptr, *S = nullptr, *R = nullptr;
     float* corr = nullptr;
     float* rowmax = nullptr;      // per frame and row: the correlation's maximum
-    float* rowsq = nullptr;       // per frame and row block: the pixels' sum of squares
+    unsigned long long* rowsq = nullptr; // per frame and row block: the pixels' sum of squares
     float2* kscratch = nullptr;   // bispectrum kernel: partial sums of split tiles
     int* ktile_cnt = nullptr;     // bispectrum kernel: parts finished per split tile
     int* shifts = nullptr;        // all frames, int2
@@ -632,7 +632,7 @@ struct smip_stack {
         CUDA_TRY(cudaMalloc(&R, sizeof(float2) * half_elems()));
         CUDA_TRY(cudaMalloc(&corr, sizeof(float) * frame_elems() * Bf));
         CUDA_TRY(cudaMalloc(&rowmax, sizeof(float) * g.H * Bf));
-        CUDA_TRY(cudaMalloc(&rowsq, sizeof(float) * row_blocks(g) * Bf));
+        CUDA_TRY(cudaMalloc(&rowsq, sizeof(*rowsq) * row_blocks(g) * Bf));
         CUDA_TRY(cudaMalloc(&ref_sq, sizeof(double)));
         if (int rc = take_err_word(&err))
             return rc;

@@ -299,23 +299,63 @@ __device__ void fft_passes(C* buf, int logn, int nl, int ls, const C* tw, int tw
     }
 }
 
-// The block's sum of v to *out (256 threads).  No barrier of its own is needed
-// after it: the next one orders the reads of the warps' sums.
-__device__ __forceinline__ void store_block_sum(float v, float* out)
+// Sums of squares of pixels, on the integer or the FP32 pipes (GB300's FP64 rate is
+// low): exact for integer frames, for floating ones a float pair (all terms are
+// positive, so no bits cancel: within 2^-40 of the exact sum).  SqSum<T> is 8 bytes.
+struct SqPair {
+    float h, l;
+};
+template <typename T> struct SqOf { using type = SqPair; };
+template <> struct SqOf<uint8_t> { using type = unsigned long long; };
+template <> struct SqOf<uint16_t> { using type = unsigned long long; };
+template <typename T> using SqSum = typename SqOf<T>::type;
+__device__ __forceinline__ void sq_add(unsigned long long& s, uint8_t v) { s += (unsigned)v * v; }
+__device__ __forceinline__ void sq_add(unsigned long long& s, uint16_t v) { s += (unsigned)v * v; }
+__device__ __forceinline__ void sq_add(SqPair& s, float v)
 {
-    __shared__ float part[8];
+    const float p = __fmul_rn(v, v);
+    df_add_lazy(s.h, s.l, p, fmaf(v, v, -p), s.h, s.l);
+}
+__device__ __forceinline__ void sq_add(SqPair& s, double v)
+{
+    const float h = (float)v, l = (float)(v - (double)h);
+    const float p = __fmul_rn(h, h);
+    df_add_lazy(s.h, s.l, p, fmaf(l, 2.f * h, fmaf(h, h, -p)), s.h, s.l);
+}
+__device__ __forceinline__ void sq_sum(unsigned long long& s, unsigned long long o) { s += o; }
+__device__ __forceinline__ void sq_sum(SqPair& s, SqPair o) { df_add_lazy(s.h, s.l, o.h, o.l, s.h, s.l); }
+__device__ __forceinline__ void sq_fold(unsigned long long& s, int o) { s += __shfl_xor_sync(0xffffffffu, s, o); }
+__device__ __forceinline__ void sq_fold(SqPair& s, int o)
+{
+    SqPair t;
+    t.h = __shfl_xor_sync(0xffffffffu, s.h, o);
+    t.l = __shfl_xor_sync(0xffffffffu, s.l, o);
+    sq_sum(s, t);
+}
+__device__ __forceinline__ double sq_value(unsigned long long s) { return (double)s; }
+__device__ __forceinline__ double sq_value(SqPair s) { return (double)s.h + (double)s.l; }
+__device__ __forceinline__ float sq_up(unsigned long long s) { return __ull2float_ru(s); }
+__device__ __forceinline__ float sq_up(SqPair s) { return __fadd_ru(s.h, s.l); }
+
+// Every warp's sum to part[8] (shared, 256 threads); after a barrier of the block,
+// the block's to *out.
+template <typename A> __device__ __forceinline__ void sq_store_warp(A s, A* part)
+{
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
-        v += __shfl_xor_sync(0xffffffffu, v, o);
+        sq_fold(s, o);
     if ((threadIdx.x & 31) == 0)
-        part[threadIdx.x >> 5] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float s = part[0];
+        part[threadIdx.x >> 5] = s;
+}
+template <typename A> __device__ __forceinline__ void sq_store_block(const A* part, A* out)
+{
+    if (threadIdx.x < 32) {
+        A s = part[threadIdx.x & 7];
 #pragma unroll
-        for (int i = 1; i < 8; ++i)
-            s += part[i];
-        *out = s;
+        for (int o = 4; o > 0; o >>= 1)
+            sq_fold(s, o);
+        if (threadIdx.x == 0)
+            *out = s;
     }
 }
 

@@ -75,11 +75,11 @@ void set_error_message(const std::string& m);
 
 // frames (dtype) -> G'(a, y) = sum_x f(x,y) exp(+2 pi i a x / W), float-float,
 // stored [f][a][y].  dtype: 0 u8, 1 u16, 2 f32, 3 f64.  rowsq[f][row_blocks(g)]:
-// FP32 sums of squares of the row blocks.  copy_out (optional, device memory):
+// sums of squares of the row blocks, 8 bytes each (SqSum, smip_dev.cuh).  copy_out (optional, device memory):
 // the frames as read, same stride.
 int row_blocks(const Geometry& g);
 cudaError_t launch_row_pass(int dtype, const void* frames, long long frame_stride_elems, int nframes,
-                            const Geometry& g, dfc* Gt, float* rowsq, const dfc* twdf, cudaStream_t st,
+                            const Geometry& g, dfc* Gt, void* rowsq, const dfc* twdf, cudaStream_t st,
                             void* copy_out = nullptr);
 
 // Column pass: S[f][a][c] = F(-a, c - H/2), power partials, and the FP32 inverse
@@ -101,8 +101,8 @@ cudaError_t launch_xcorr_rows(const float2* T, float* corr, float* rowmax, int n
 // refsq: those of the reference, or null: *ref_sq (device) holds its sum.
 // first: frame 0 is the reference (refsq is given), *ref_sq is written.
 cudaError_t launch_xcorr_shift(int dtype, const float* corr, const float* rowmax, const void* frames,
-                               long long frame_stride_elems, const void* ref, const float* rowsq, int nsq,
-                               const float* refsq, double* ref_sq, int nframes, int first, const Geometry& g,
+                               long long frame_stride_elems, const void* ref, const void* rowsq, int nsq,
+                               const void* refsq, double* ref_sq, int nframes, int first, const Geometry& g,
                                int* shifts, cudaStream_t st);
 
 // sum += |frames| shifted back by their shifts (Array2::shifted semantics);
@@ -114,7 +114,7 @@ cudaError_t launch_saa_add(int dtype, void* sum, const void* frames, long long f
 // (k_fftg.cu); same inputs and outputs, twiddles from the stack's GenTw tables.
 int gen_row_blocks(const Geometry& g);
 cudaError_t launch_gen_row_pass(int dtype, const void* frames, long long fstride, int nframes, const Geometry& g,
-                                dfc* Gt, float* rowsq, const dfc* twW, cudaStream_t st, void* copy_out = nullptr);
+                                dfc* Gt, void* rowsq, const dfc* twW, cudaStream_t st, void* copy_out = nullptr);
 cudaError_t launch_gen_col_pass(const dfc* Gt, float2* S, float2* Rbuf, float2* T, double* Ppart, int nframes, int fpc,
                                 int first, const Geometry& g, const dfc* twH, const float2* twH32, cudaStream_t st);
 cudaError_t launch_gen_xcorr_rows(const float2* T, float* corr, float* rowmax, int nframes, const Geometry& g,

@@ -54,7 +54,7 @@ constexpr size_t kOffC = kOffP + align256(kHalf * sizeof(double));       // corr
 constexpr size_t kOffM = kOffC + align256((size_t)kMaxN * kMaxN * sizeof(float)); // row maxima
 constexpr size_t kOffQ = kOffM + align256((size_t)kMaxN * sizeof(float));          // sums of squares, 2 frames
 constexpr int kTw = 1 << (kTwLog - 1);
-constexpr size_t kOffTw = kOffQ + align256(2 * (size_t)kMaxN * sizeof(float));     // FP32 twiddles
+constexpr size_t kOffTw = kOffQ + align256(2 * (size_t)kMaxN * sizeof(unsigned long long));    // FP32 twiddles
 constexpr size_t kOffTwDf = kOffTw + align256(kTw * sizeof(float2));     // float-float twiddles
 constexpr size_t kOffWarm = kOffTwDf + align256(kTw * sizeof(dfc));     // warm-up frame (16 x 16 doubles, zero)
 constexpr size_t kWarmN = 16;
@@ -145,7 +145,7 @@ cudaError_t run_shift(unsigned char* base, const double* ref, const double* fram
     double* Pp = reinterpret_cast<double*>(base + kOffP);
     float* corr = reinterpret_cast<float*>(base + kOffC);
     float* rowmax = reinterpret_cast<float*>(base + kOffM);
-    float* rowsq = reinterpret_cast<float*>(base + kOffQ);
+    unsigned long long* rowsq = reinterpret_cast<unsigned long long*>(base + kOffQ);
     const int nsq = row_blocks(g);
     const float2* tw = reinterpret_cast<const float2*>(base + kOffTw);
     const dfc* twdf = reinterpret_cast<const dfc*>(base + kOffTwDf);
