@@ -12,7 +12,7 @@
 // to the lowest linear index (std::max_element's first maximum).  The bound
 // is 8 * 2^-24 * log2(W*H) * ||ref||_2 * ||frame||_2 * W*H, a few times the
 // worst-case error of an FP32 radix-2 FFT convolution (for mixed-radix
-// transforms the odd factors of W and H count themselves instead of their log2).
+// transforms the odd factors of W and H count themselves, and factors of 2 twice).
 #include <cstdint>
 
 #include "smip_dev.cuh"
@@ -395,14 +395,13 @@ cudaError_t launch_xcorr_shift(int dtype, const float* corr, const float* rowmax
                                int nframes, int first, const Geometry& g, int* shifts, cudaStream_t st)
 {
     // the correlation's FP32 error grows with the transforms' stages: log2(W H)
-    // radix-2 stages; on the generic path log2 of the factors 2, 4 and 8
-    // (radix-2 stages in registers) and the sum of the odd ones (each pass a sum
-    // of that many terms)
+    // radix-2 stages; on the generic path two for each factor of 2 and the odd
+    // factors themselves (a radix-R pass is a sum of R terms, or fewer roundings)
     const int logW = g.generic ? -1 : g.logW;
     double stages = g.logW + g.logH;
     if (g.generic) {
         stages = 0.0;
-        auto of = [](int R) { return R == 2 ? 1 : R == 4 ? 2 : R == 8 ? 3 : R; };
+        auto of = [](int R) { return R == 8 ? 6 : R; };
         for (int k = 0; k < g.pW.nf; ++k) stages += of(g.pW.fac[k]);
         for (int k = 0; k < g.pH.nf; ++k) stages += of(g.pH.fac[k]);
     }
