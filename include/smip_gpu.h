@@ -265,7 +265,8 @@ SMIP_GPU_API int smip_xcorr_displacement(int device, const double* ref, const do
  * (a cudaStream_t, or NULL for the default stream).  Allocates nothing: all
  * intermediates live in one fixed ~3 MB device array inside the library, so
  * ncols and nrows must be powers of two in [16, 256] (SMIP_E_UNSUPPORTED
- * otherwise).  The first call on a device looks up that array and uploads
+ * otherwise).  The pointers must be aligned to their elements
+ * (SMIP_E_INVALID_ARGUMENT otherwise, before anything runs on the device).  The first call on a device looks up that array and uploads
  * constants, so make it before any stream capture.  Calls share the array:
  * calls that overlap on the GPU race and must be ordered by the caller. */
 SMIP_GPU_API int smip_xcorr_displacement_noalloc(const double* ref, const double* frame, long ncols, long nrows,

@@ -151,16 +151,10 @@ cudaError_t run_shift(unsigned char* base, const double* ref, const double* fram
     const dfc* twdf = reinterpret_cast<const dfc*>(base + kOffTwDf);
     const long long n = (long long)ncols * nrows;
     // reference and frame as a batch of two: two launches to the spectra and the
-    // correlation's columns, two to the shift.  The frames are one stride apart
-    // when their distance is a whole number of pixels.
-    cudaError_t e;
-    const long long apart = reinterpret_cast<const char*>(frame) - reinterpret_cast<const char*>(ref);
-    if (apart % (long long)sizeof(double) == 0) {
-        e = launch_row_pass(SMIP_F64, ref, apart / (long long)sizeof(double), 2, g, Gt, rowsq, twdf, st);
-    } else {
-        e = launch_row_pass(SMIP_F64, ref, n, 1, g, Gt, rowsq, twdf, st);
-        if (e == cudaSuccess) e = launch_row_pass(SMIP_F64, frame, n, 1, g, Gt + half, rowsq + nsq, twdf, st);
-    }
+    // correlation's columns, two to the shift.  They are one stride apart, which
+    // may be negative or zero; both are aligned, so it is a whole number of pixels.
+    const long long apart = (reinterpret_cast<intptr_t>(frame) - reinterpret_cast<intptr_t>(ref)) / (long long)sizeof(double);
+    cudaError_t e = launch_row_pass(SMIP_F64, ref, apart, 2, g, Gt, rowsq, twdf, st);
     if (e == cudaSuccess) e = launch_col_pass(Gt, S, R, T, Pp, 2, 16, 1, g, twdf, tw, st);
     if (e == cudaSuccess) e = launch_xcorr_rows(T + half, corr, rowmax, 1, g, tw, st);
     if (e == cudaSuccess)
@@ -178,6 +172,9 @@ extern "C" int smip_xcorr_displacement_noalloc(const double* ref, const double* 
     if (!pow2_in(ncols) || !pow2_in(nrows))
         return fail(SMIP_E_UNSUPPORTED, "smip_xcorr_displacement_noalloc: ncols and nrows must be powers of two in "
                                         "[16, 256] (the fixed scratch array holds frames up to 256 x 256)");
+    auto aligned = [](const void* p, size_t a) { return reinterpret_cast<uintptr_t>(p) % a == 0; };
+    if (!aligned(ref, sizeof(double)) || !aligned(frame, sizeof(double)) || !aligned(shift, sizeof(int)))
+        return fail(SMIP_E_INVALID_ARGUMENT, "device pointer not aligned to its elements");
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess)
         return fail(SMIP_E_CUDA, "cudaGetDevice failed");
