@@ -116,6 +116,14 @@ SMIP_GPU_API int smip_stack_set_kernel_config(smip_stack_t s, int variant, int m
 #define SMIP_RECO_RINGS 1
 SMIP_GPU_API int smip_stack_set_reco_mode(smip_stack_t s, int mode);
 
+/* Thread blocks of the spiral walk, each on an SM of its own: 0 (default)
+ * takes two below depth 28, four below 40 and eight from there on, the fewest
+ * that keep its serial part busy; 1, 2, 4 or 8 asks for as many (fewer leave
+ * more of the GPU to other jobs; one sums a point's pairs beside the serial
+ * part and is the slowest).  Where the GPU places no such cluster the walk
+ * takes a smaller one.  Results do not depend on it, to the bit. */
+SMIP_GPU_API int smip_stack_set_walk_ctas(smip_stack_t s, int ctas);
+
 /* Replaces Bispectrum::accumulate_from_fft(const Array2<complex<double>>&)
  * (bispectrum.h:82-83, 356-409) for spectra computed elsewhere: count spectra
  * of ncols x nrows complex<double> in FFT order, host or device memory.
@@ -191,6 +199,12 @@ SMIP_GPU_API int smip_stack_reconstruct(smip_stack_t s, double reco_radius, doub
  * as above (pre-window phases, as reconstruct_phases returns them). */
 SMIP_GPU_API int smip_stack_finish(smip_stack_t s, double reco_radius, double* image, double* phases,
                                    unsigned char* flags, double* consistency);
+
+/* Number of pairs that the last reconstruction formed each point's phase from
+ * (the divisor of its mean phasor, phasereco.h:110-122): ncols*nrows ints in
+ * FFT order, -1 at the seeds, 0 where there is no phase.  SMIP_E_BAD_CALL
+ * before the first one, also after a reset. */
+SMIP_GPU_API int smip_stack_reco_counts(smip_stack_t s, int* counts);
 
 /* Allocates the reconstruction's device buffers and builds its spiral visit
  * tables for reco_radius ahead of smip_stack_reconstruct / smip_stack_finish

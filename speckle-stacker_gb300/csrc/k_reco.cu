@@ -1317,7 +1317,8 @@ cudaError_t launch_offset_probe(const Geometry& g, const int* idx, long long n, 
     return cudaGetLastError();
 }
 
-cudaError_t launch_phase_reco(const RecoJob* jobs_dev, int njobs, int max_W, int max_H, int max_De, cudaStream_t st)
+cudaError_t launch_phase_reco(const RecoJob* jobs_dev, int njobs, int max_W, int max_H, int max_De, int ctas,
+                              cudaStream_t st)
 {
     const int nv = (max_De + 1) * (max_De + 1), nslots = (nv + 31) / 32 * 32;
     spiral_plan_kernel<<<dim3(1216, njobs), 32 * kPlanWarps, sizeof(int) * nslots, st>>>(jobs_dev);
@@ -1326,7 +1327,7 @@ cudaError_t launch_phase_reco(const RecoJob* jobs_dev, int njobs, int max_W, int
     // another shape must never lower it under this one)
     const int smem_max = (int)(box_bytes(kMaxWords * 32) + (size_t)kRowWords * 256 * (kRecoThreads / 32));
     size_t smem = walk_smem(max_De, nslots, true);
-    int ncta = walk_ctas(max_De);
+    int ncta = ctas ? ctas : walk_ctas(max_De);
     cudaError_t e = cudaSuccess;
     if (ncta > 1) {
         // a cluster per job, or the largest that the GPU can place

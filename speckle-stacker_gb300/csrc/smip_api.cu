@@ -315,6 +315,7 @@ struct Reco {
     double R = -1.0;
     int2* visits = nullptr;
     int mode = 0;                 // 0: the reference's spiral walk; 1: ring-parallel estimator
+    int ctas = 0;                 // of the walk (0: by depth)
     int* fring = nullptr;         // ring mode: per point the ring that set its phase (-1: none)
     int* rq = nullptr;            // ring mode: visit indices grouped by ring
     std::vector<int> roff;        // ring k: rq[roff[k] .. roff[k+1])
@@ -450,7 +451,7 @@ struct Reco {
         if (mode == 1) {
             CUDA_TRY(launch_ring_reco(job, fring, rq, roff, g.W, g.H, st));
         } else {
-            CUDA_TRY(launch_phase_reco(job, 1, g.W, g.H, g.De, st));
+            CUDA_TRY(launch_phase_reco(job, 1, g.W, g.H, g.De, ctas, st));
         }
         return SMIP_OK;
     }
@@ -548,6 +549,7 @@ struct smip_stack {
     long shifts_cap = 0;
     int* err = nullptr;
     Reco reco;
+    bool reco_done = false;       // reco holds a reconstruction
     double2* Z = nullptr;
     double* pfull = nullptr;
     double* maxbuf = nullptr;
@@ -1017,6 +1019,17 @@ extern "C" int smip_stack_set_reco_mode(smip_stack_t s, int mode)
     return SMIP_OK;
 }
 
+extern "C" int smip_stack_set_walk_ctas(smip_stack_t s, int ctas)
+{
+    int rc = check_stack(s);
+    if (rc)
+        return rc;
+    if (ctas != 0 && ctas != 1 && ctas != 2 && ctas != 4 && ctas != 8)
+        return fail(SMIP_E_INVALID_ARGUMENT, "a phase walk runs as 1, 2, 4 or 8 CTAs (0: by depth)");
+    s->reco.ctas = ctas; // read on the host when the next reconstruction is issued
+    return SMIP_OK;
+}
+
 extern "C" int smip_stack_accumulate_fft(smip_stack_t s, const double* spectra, long count, int on_device)
 {
     int rc = check_stack(s);
@@ -1066,6 +1079,7 @@ extern "C" int smip_stack_reset(smip_stack_t s)
     s->nframes = 0;
     s->pending = 0;
     s->has_ref = false;
+    s->reco_done = false;
     s->mode = 0;
     return SMIP_OK;
 }
@@ -1448,7 +1462,10 @@ static int stack_reco(smip_stack_t s, double R, bool image)
         return fail(SMIP_E_DOMAIN, "WindowFunction aperture size <= 0");
     if ((rc = prepare_reco(s, R)) || (rc = normalize_bispec(s, s->rst)))
         return rc;
-    return s->reco.run(s->Bn, R, s->err, s->rst);
+    if ((rc = s->reco.run(s->Bn, R, s->err, s->rst)))
+        return rc;
+    s->reco_done = true;
+    return SMIP_OK;
 }
 
 static int rejoin_stream(smip_stack_t s)
@@ -1485,6 +1502,25 @@ extern "C" int smip_stack_finish(smip_stack_t s, double R, double* image, double
     if ((rc = s->reco.download(phases, flags, cons, s->st)))
         return rc;
     return check_dev_err(s->err, s->st);
+}
+
+extern "C" int smip_stack_reco_counts(smip_stack_t s, int* counts)
+{
+    int rc = check_stack(s);
+    if (rc)
+        return rc;
+    if (!counts)
+        return fail(SMIP_E_INVALID_ARGUMENT, "null output");
+    if (!s->reco_done)
+        return fail(SMIP_E_BAD_CALL, "the stack holds no phase reconstruction");
+    const size_t n = s->frame_elems();
+    std::vector<unsigned char> fl(n);
+    CUDA_TRY(cudaMemcpyAsync(counts, s->reco.cnt, sizeof(int) * n, cudaMemcpyDeviceToHost, s->st));
+    CUDA_TRY(cudaMemcpyAsync(fl.data(), s->reco.flags, n, cudaMemcpyDeviceToHost, s->st));
+    CUDA_TRY(cudaStreamSynchronize(s->st));
+    for (size_t p = 0; p < n; ++p)
+        counts[p] = fl[p] ? counts[p] : 0;
+    return SMIP_OK;
 }
 
 extern "C" int smip_stack_prepare_reco(smip_stack_t s, double reco_radius)

@@ -189,7 +189,9 @@ constexpr int kRecoLag = 32;     // visits between a point's phase and the paral
 constexpr int kRecentMax = 64;   // recent pairs per visit: at most 32 by u and 32 by v
 // pair slots of a plan row: (De+1)^2 rounded up to whole warps (16-byte aligned rows)
 constexpr size_t plan_row(int De) { return ((size_t)(De + 1) * (De + 1) + 31) / 32 * 32; }
-cudaError_t launch_phase_reco(const RecoJob* jobs_dev, int njobs, int max_W, int max_H, int max_De, cudaStream_t st);
+// ctas: of a job's walk (1, 2, 4 or 8; 0: by depth).
+cudaError_t launch_phase_reco(const RecoJob* jobs_dev, int njobs, int max_W, int max_H, int max_De, int ctas,
+                              cudaStream_t st);
 // Ring-parallel estimator (opt-in, not the reference's): rq holds the spiral's
 // visit indices grouped by ring, ring k at [roff[k], roff[k+1]); fring: W*H ints.
 cudaError_t launch_ring_reco(const RecoJob* job_dev, int* fring, const int* rq, const std::vector<int>& roff, int W,

@@ -229,6 +229,7 @@ public:
                                 r.pm.consistency.data()));
         return r;
     }
+    void set_walk_ctas(int ctas) const { check(smip_stack_set_walk_ctas(handle(), ctas)); }
     // buffers and visit tables of finish(reco_radius) ahead of the first call
     void prepare_reco(double reco_radius) const { check(smip_stack_prepare_reco(handle(), reco_radius)); }
     void write_to_file(const std::string& path) const { check(smip_stack_save_bispectrum(handle(), path.c_str())); }

@@ -125,6 +125,8 @@ def _load():
         "smip_xcorr_displacement_noalloc": ([vp, vp, C.c_long, C.c_long, vp, vp], C.c_int),
         "smip_stack_reset": ([vp], C.c_int),
         "smip_stack_set_reco_mode": ([vp, C.c_int], C.c_int),
+        "smip_stack_set_walk_ctas": ([vp, C.c_int], C.c_int),
+        "smip_stack_reco_counts": ([vp, ip], C.c_int),
         "smip_stack_set_timing": ([vp, C.c_int], C.c_int),
         "smip_stack_kernel_time": ([vp, dp, lp, dp], C.c_int),
         "smip_kernel_launches": ([], C.c_longlong),
@@ -283,6 +285,11 @@ class Stack:
         m = {"spiral": 0, "rings": 1}.get(mode, mode)
         _check(_L().smip_stack_set_reco_mode(self._h, int(m)))
 
+    def set_walk_ctas(self, ctas: int = 0):
+        """Thread blocks of the spiral walk: 1, 2, 4 or 8 (0: by depth).  Fewer
+        leave more of the GPU to other jobs; the results are the same bits."""
+        _check(_L().smip_stack_set_walk_ctas(self._h, int(ctas)))
+
     def reset(self):
         """Zero the accumulators for a new job (device buffers are kept)."""
         _check(_L().smip_stack_reset(self._h))
@@ -346,6 +353,13 @@ class Stack:
                                            _p(fl, C.c_ubyte), _p(cs, C.c_double)))
         s = (self.nrows, self.ncols)
         return ph.reshape(s), fl.reshape(s), cs.reshape(s)
+
+    def reco_counts(self):
+        """Pairs that the last reconstruction formed each point's phase from
+        (-1: a seed, 0: no phase)."""
+        out = np.zeros((self.nrows, self.ncols), np.int32)
+        _check(_L().smip_stack_reco_counts(self._h, _p(out, C.c_int)))
+        return out
 
     def finish(self, reco_radius: float):
         """(image, phases, flags, consistency) of main.cpp:318-376."""
