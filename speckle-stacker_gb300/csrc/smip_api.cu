@@ -104,33 +104,53 @@ std::map<int, DeviceCtx> g_ctx;
 // Device error words.  They lie in page-locked host memory that the kernels
 // write through (record_error, on a failure only), so that a result call reads
 // one after its own wait instead of copying it: a copy of four bytes and its
-// wait cost about 10 us, four times a job.  Pages are made as they are needed
-// and kept; a stack takes a word and gives it back.
+// wait cost about 10 us, four times a job.  A stack takes a word, a cache line of
+// its own, and gives it back; a page that has no word taken is freed, but for the
+// last one (4 KB).
+struct ErrPage {
+    int* base;
+    uint64_t free; // a bit per word
+};
+constexpr int kErrStep = 64 / (int)sizeof(int), kErrWords = 64;
 std::mutex g_err_mu;
-std::vector<int*> g_err_free;
+std::vector<ErrPage> g_err_pages;
 
 int take_err_word(int** out)
 {
     std::lock_guard<std::mutex> lk(g_err_mu);
-    if (g_err_free.empty()) {
-        int* page = nullptr;
-        constexpr int kStep = 64 / (int)sizeof(int), kWords = 64; // a cache line each
-        CUDA_TRY(cudaHostAlloc(&page, (size_t)kWords * kStep * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped));
-        for (int i = 0; i < kWords; ++i)
-            g_err_free.push_back(page + i * kStep);
+    auto pg = std::find_if(g_err_pages.begin(), g_err_pages.end(), [](const ErrPage& p) { return p.free != 0; });
+    if (pg == g_err_pages.end()) {
+        ErrPage p { nullptr, ~0ull };
+        CUDA_TRY(cudaHostAlloc(&p.base, (size_t)kErrWords * kErrStep * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped));
+        g_err_pages.push_back(p);
+        pg = g_err_pages.end() - 1;
     }
-    *out = g_err_free.back();
-    g_err_free.pop_back();
+    int w = 0;
+    while (!(pg->free >> w & 1))
+        ++w;
+    pg->free &= ~(1ull << w);
+    *out = pg->base + w * kErrStep;
     **out = 0;
     return SMIP_OK;
 }
 
+// (no kernel that might write the word is in flight)
 void give_err_word(int* w)
 {
     if (!w)
         return;
     std::lock_guard<std::mutex> lk(g_err_mu);
-    g_err_free.push_back(w);
+    for (size_t k = 0; k < g_err_pages.size(); ++k) {
+        ErrPage& p = g_err_pages[k];
+        if (w < p.base || w >= p.base + kErrWords * kErrStep)
+            continue;
+        p.free |= 1ull << ((w - p.base) / kErrStep);
+        if (p.free == ~0ull && g_err_pages.size() > 1) {
+            cudaFreeHost(p.base);
+            g_err_pages.erase(g_err_pages.begin() + k);
+        }
+        return;
+    }
 }
 
 int device_ctx(int dev, DeviceCtx** out)
