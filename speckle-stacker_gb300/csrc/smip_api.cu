@@ -42,9 +42,11 @@ static int fail(int code, const std::string& msg)
 #define CUDA_TRY(expr)                                                                                     \
     do {                                                                                                   \
         cudaError_t e_ = (expr);                                                                           \
-        if (e_ != cudaSuccess)                                                                             \
+        if (e_ != cudaSuccess) {                                                                           \
+            cudaGetLastError(); /* reported here, not by the next launch */                                \
             return fail(e_ == cudaErrorMemoryAllocation ? SMIP_E_NO_MEMORY : SMIP_E_CUDA,                  \
                         std::string(#expr) + ": " + cudaGetErrorString(e_));                               \
+        }                                                                                                  \
     } while (0)
 
 extern "C" const char* smip_last_error(void) { return g_last_error.c_str(); }
@@ -376,7 +378,8 @@ struct Reco {
     int prepare(double radius, cudaStream_t st)
     {
         const size_t np = (size_t)g.W * g.H;
-        if (!phases) {
+        if (!pmap) { // the last of them (each is freed before it is taken again)
+            dfree(phases), dfree(phf), dfree(sums), dfree(cnt), dfree(cons), dfree(flags), dfree(job), dfree(oor);
             CUDA_TRY(cudaMalloc(&phases, sizeof(double2) * np));
             CUDA_TRY(cudaMalloc(&phf, sizeof(float2) * np));
             CUDA_TRY(cudaMalloc(&sums, sizeof(float4) * np));
@@ -391,6 +394,7 @@ struct Reco {
             std::vector<int> vring;
             std::vector<int2> v = reco_visits(radius, &vring);
             CUDA_TRY(cudaStreamSynchronize(st));
+            R = -1.0; // until the new tables are complete: a failure below leaves none
             dfree(rq);
             {   // ring lists: each point once per ring, in visit order
                 const int nr = vring.empty() ? 1 : vring.back() + 1;
