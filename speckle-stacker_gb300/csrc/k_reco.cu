@@ -384,7 +384,14 @@ constexpr int kRing = 64;
 constexpr int kMaxParts = 6;
 constexpr int kStep = 4;                 // visits between two looks of the serial warp at the other warps
 constexpr int kGroups = kRing / kStep;
-constexpr int kRowWords = 40;            // words of a plan row that a summing warp of a cluster keeps in shared memory
+// Words of a plan row that a summing warp of a cluster keeps in shared memory.  The
+// function's limit is one number: the box of the largest depth, 16 warps' rows of
+// 40 words and the static arrays take 226 of 227 KB.  Only depths 36 and 38 have
+// longer parts (43, 48 words in one part; 39 at depth 34, 18 in three at 40) and
+// read their rows from global memory: 411 and 420 ns a visit at 144 x 144, R = 64
+// (254 at depths 34 and 40).  With rows of 48 words and a limit of these depths'
+// own they took 270 and 275 at 128 x 128 (373 and 378 without).
+constexpr int kRowWords = 40;
 constexpr unsigned long long kRecoWaitNs = 2000000000ull;
 static_assert(kRing > kRecoLag + 8, "ring slots outlive the lag and the serial warp's look-ahead");
 
@@ -931,7 +938,9 @@ __global__ void __launch_bounds__(kRecoThreads, 1) phase_walk_kernel(const RecoJ
         const int wb = part * nwords / nparts, we = (part + 1) * nwords / nparts;
         // In a cluster a visit's plan row comes into shared memory before the
         // visit may be summed, and only the gathers of u stand between the
-        // progress and the sum: kB of them a lane in flight (2 registers each).
+        // progress and the sum: kB of them a lane in flight (2 registers each), in
+        // batches of equal length (10, 18 or 20 words compiled; 7, 9 or 12 at a time
+        // were slower at depths 24, 32 and 48).
         constexpr int kB = 20, kBDirect = 10;
         const int nbat = (we - wb + kB - 1) / kB, nbw = (we - wb + nbat - 1) / nbat; // batches, words of one
         const bool staged = MULTI && part_words(De, nwords) <= kRowWords;
