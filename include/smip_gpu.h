@@ -154,8 +154,9 @@ SMIP_GPU_API int smip_batch_launch(smip_stack_t* stacks, long count);
 
 /* smip_batch_launch with reserve_sms streaming multiprocessors left out of
  * the persistent grid (0 <= reserve_sms < SM count; 0 is smip_batch_launch),
- * so that phase recoveries of stacks launched earlier -- one block each, on
- * their high-priority streams -- run beside the launch instead of after it.
+ * so that phase recoveries of stacks launched earlier -- one to eight blocks
+ * each, on their high-priority streams -- run beside the launch instead of
+ * after it.
  * One graph is kept per grid size.  Results do not depend on reserve_sms. */
 SMIP_GPU_API int smip_batch_launch_reserve(smip_stack_t* stacks, long count, int reserve_sms);
 

@@ -164,19 +164,11 @@ template <int R, typename C>
 __device__ __forceinline__ void stockham_pass(const C* x, C* y, int L, int Ns, const unsigned* mp, int nl, int ls,
                                               const C* tw, int sign)
 {
-    const int LR = L / R, step = LR / Ns;
+    const int LR = L / R;
     for (int idx = threadIdx.x; idx < nl * LR; idx += blockDim.x) {
         const int line = idx / LR, j = idx - line * LR;
-        int k1, o0; // twiddle exponent of r = 1; first output
-        if (mp) { // precomputed for this length: no divisions
-            const unsigned m = __ldg(mp + j);
-            o0 = (int)(m & 0xffffu);
-            k1 = (int)(m >> 16);
-        } else {
-            const int k = j % Ns;
-            o0 = (j - k) * R + k;
-            k1 = k * step;
-        }
+        const unsigned m = __ldg(mp + j); // first output, twiddle exponent of r = 1: no divisions
+        const int o0 = (int)(m & 0xffffu), k1 = (int)(m >> 16);
         const C* X = x + line * ls + j;
         C v[R];
         v[0] = X[0];
@@ -209,7 +201,7 @@ __device__ C* stockham(C* x, C* y, const GenPlan& p, int nl, int ls, const C* tw
     int Ns = 1;
     for (int f = 0; f < p.nf; ++f) {
         const int R = p.fac[f];
-        const unsigned* mp = p.map ? p.map + f * L : nullptr;
+        const unsigned* mp = p.map + f * L;
         switch (R) {
         case 2: stockham_pass<2>(x, y, L, Ns, mp, nl, ls, tw, sign); break;
         case 3: stockham_pass<3>(x, y, L, Ns, mp, nl, ls, tw, sign); break;
@@ -218,20 +210,11 @@ __device__ C* stockham(C* x, C* y, const GenPlan& p, int nl, int ls, const C* tw
         case 7: stockham_pass<7>(x, y, L, Ns, mp, nl, ls, tw, sign); break;
         case 8: stockham_pass<8>(x, y, L, Ns, mp, nl, ls, tw, sign); break;
         default: { // a larger prime: one output per thread
-            const int LR = L / R, step = LR / Ns; // L / (Ns R)
+            const int LR = L / R;
             for (int idx = threadIdx.x; idx < nl * L; idx += blockDim.x) {
                 const int line = idx / L, o = idx - line * L;
-                int j, e0;
-                if (mp) { // precomputed for this length: no divisions
-                    const unsigned m = __ldg(mp + o);
-                    j = (int)(m & 0xffffu);
-                    e0 = (int)(m >> 16);
-                } else {
-                    const int k = o % Ns, t = o / Ns;
-                    const int q = t % R;
-                    j = (t / R) * Ns + k;
-                    e0 = (k + q * Ns) * step; // < L
-                }
+                const unsigned m = __ldg(mp + o); // first input, exponent step
+                const int j = (int)(m & 0xffffu), e0 = (int)(m >> 16);
                 const C* X = x + line * ls + j;
                 C acc = X[0];
                 int e = 0;

@@ -26,7 +26,7 @@ struct GenPlan {
     int L;
     int nf;
     int fac[kMaxFactors];
-    // per pass f, nf x L entries in device memory (null: computed): a butterfly
+    // per pass f, nf x L entries in device memory (the stack's): a butterfly
     // j's first output | twiddle exponent << 16, or for a larger prime an output
     // o's input index j | twiddle exponent step << 16 (k_fftg.cu)
     const unsigned* map = nullptr;
