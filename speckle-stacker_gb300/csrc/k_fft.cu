@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(256, 4) row_pass_kernel(const T* __restrict__ 
 {
     extern __shared__ dfc smdf[];
     __shared__ SqSum<T> sqpart[8];
-    SqSum<T> sq {}; // of this thread's pixels, for the correlation's error bound (k_xcorr.cu)
+    SqLane<T> sq {}; // of this thread's pixels, for the correlation's error bound (k_xcorr.cu)
     const int W = 1 << logW;
     dfc* tw = smdf;                                // W - 1, stage-packed (+1 spare)
     dfc* lines = smdf + W;                         // [kRowBlock/2][pad8(W) + 1]

@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(256, 4) gen_row_kernel(const T* __restrict__ f
 {
     extern __shared__ dfc smg[];
     __shared__ SqSum<T> sqpart[8];
-    SqSum<T> sq {}; // of this thread's pixels, for the correlation's error bound (k_xcorr.cu)
+    SqLane<T> sq {}; // of this thread's pixels, for the correlation's error bound (k_xcorr.cu)
     const int W = pw.L;
     dfc* tw = smg;
     dfc* X = tw + W;

@@ -309,8 +309,12 @@ template <typename T> struct SqOf { using type = SqPair; };
 template <> struct SqOf<uint8_t> { using type = unsigned long long; };
 template <> struct SqOf<uint16_t> { using type = unsigned long long; };
 template <typename T> using SqSum = typename SqOf<T>::type;
-__device__ __forceinline__ void sq_add(unsigned long long& s, uint8_t v) { s += (unsigned)v * v; }
-__device__ __forceinline__ void sq_add(unsigned long long& s, uint16_t v) { s += (unsigned)v * v; }
+// a thread's own sum: 32 bits for bytes (at most 2^12 of them a warp)
+template <typename T> struct SqLaneOf { using type = SqSum<T>; };
+template <> struct SqLaneOf<uint8_t> { using type = unsigned; };
+template <typename T> using SqLane = typename SqLaneOf<T>::type;
+__device__ __forceinline__ void sq_add(unsigned& s, uint8_t v) { s += (unsigned)v * v; }
+__device__ __forceinline__ void sq_add(unsigned long long& s, uint16_t v) { s += (unsigned long long)v * v; }
 __device__ __forceinline__ void sq_add(SqPair& s, float v)
 {
     const float p = __fmul_rn(v, v);
@@ -339,6 +343,12 @@ __device__ __forceinline__ float sq_up(SqPair s) { return __fadd_ru(s.h, s.l); }
 
 // Every warp's sum to part[8] (shared, 256 threads); after a barrier of the block,
 // the block's to *out.
+__device__ __forceinline__ void sq_store_warp(unsigned s, unsigned long long* part)
+{
+    s = __reduce_add_sync(0xffffffffu, s);
+    if ((threadIdx.x & 31) == 0)
+        part[threadIdx.x >> 5] = s;
+}
 template <typename A> __device__ __forceinline__ void sq_store_warp(A s, A* part)
 {
 #pragma unroll
