@@ -60,7 +60,7 @@ cudaError_t launch_bounded_wait_probe(int* err, const int* never, double timeout
 // ------------------------------------------------------- normalise, merge
 // (B - C) / n as FP64 arithmetic and one rounding give it, to the bit, but on the
 // FP32 pipes (GB300's FP64 rate bound this kernel: 351 us at 256 x 256, d = 32,
-// 1.3 TB/s; now HBM does).  The difference is an exact float pair, its product
+// 1.3 TB/s; now 63 us, 7.1 TB/s of algorithmic bytes).  The difference is an exact float pair, its product
 // with 1/n as a float pair is within 2^-45 of FP64's.  Where that leaves the
 // rounding open (a value that close to the middle of two floats), and for values
 // so small that the pair loses bits, infinities and NaN, the FP64 form decides.

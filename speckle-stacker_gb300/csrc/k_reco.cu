@@ -327,8 +327,8 @@ __global__ void __launch_bounds__(32 * kPlanWarps) spiral_plan_kernel(const Reco
     }
 }
 
-// The walk: one cluster of CTAs per job (or one CTA, where the GPU places no
-// cluster).
+// The walk: one cluster of CTAs per job (or one CTA, where the caller asks for it
+// or the GPU places no cluster).
 //   warp 0 of rank 0 (the serial warp) runs the visits in order;
 //   the writer, on another sub-partition, copies what the serial warp found
 //     into the phase map in global memory and publishes the progress, first to
@@ -455,7 +455,8 @@ static size_t walk_smem(int De, int nslots, bool multi)
 // CTAs per job: as few as keep the serial warp busy, because jobs that share
 // the GPU need the other SMs.  Cycles a visit with 2 / 4 / 8 CTAs: 459 / 456 /
 // 455 at depth 24, 528 / 440 / 435 at depth 32; with 4 / 8: 479 / 428 at depth 48.
-// (A lone CTA, where no cluster can be placed: 1,054 at depth 24, 1,241 at 32.)
+// (A lone CTA, asked for or where no cluster can be placed: 1,108 and 1,240 at
+// depths 24 and 32, the whole call.)
 static int walk_ctas(int De) { return De < 28 ? 2 : (De < kPartsDepth ? 4 : 8); }
 
 template <bool MULTI> // a cluster of CTAs per job, or one CTA

@@ -173,7 +173,7 @@ template <typename T> __device__ __forceinline__ bool norm_ok(float s) { return 
 // Bound by latency: a frame's pixels are read only where more than one position
 // lies within the bound of the peak (few frames), and the norms come from the row
 // pass.  With the frame read for its norm and the peak always re-scored, 2000
-// frames of 256 x 256 took 369 us instead of 102.
+// frames of 256 x 256 took 369 us instead of 99.
 // One CTA per frame.  rowsq: nsq sums per frame; refsq: those of the reference,
 // or null (its sum of squares is *ref_sq then).  The stack's frame 0 (first) is
 // the reference itself: it shifts by (0, 0), and its CTA writes *ref_sq for the
