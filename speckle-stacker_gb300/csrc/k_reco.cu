@@ -386,11 +386,12 @@ constexpr int kStep = 4;                 // visits between two looks of the seri
 constexpr int kGroups = kRing / kStep;
 // Words of a plan row that a summing warp of a cluster keeps in shared memory.  The
 // function's limit is one number: the box of the largest depth, 16 warps' rows of
-// 40 words and the static arrays take 226 of 227 KB.  Only depths 36 and 38 have
-// longer parts (43, 48 words in one part; 39 at depth 34, 18 in three at 40) and
-// read their rows from global memory: 411 and 420 ns a visit at 144 x 144, R = 64
-// (254 at depths 34 and 40).  With rows of 48 words and a limit of these depths'
-// own they took 270 and 275 at 128 x 128 (373 and 378 without).
+// 40 words and the static arrays take 225,168 of 232,448 bytes; 43 words would not
+// fit.  Only depths 36 and 38 have longer parts (43, 48 words in one part; 39 at
+// depth 34, 18 in three at 40) and read their rows from global memory: 411 and 420
+// ns a visit at 144 x 144, R = 64 (254 at depths 34 and 40).  With rows of 48 words
+// and a limit of these depths' own they took 270 and 275 at 128 x 128 (373 and 378
+// without).
 constexpr int kRowWords = 40;
 constexpr unsigned long long kRecoWaitNs = 2000000000ull;
 static_assert(kRing > kRecoLag + 8, "ring slots outlive the lag and the serial warp's look-ahead");
